@@ -102,3 +102,76 @@ def test_cuda_graph_decode_matches_eager_decode():
     assert agree >= len(want) - 1, (got, want)
     for g, w in zip(got, want):
         assert g[:6] == w[:6]
+
+
+# (keys before the portion, its tokens): tile edges (128 keys, 128 / 256 query rows) and their neighbours, the smallest portions
+@pytest.mark.parametrize("Hq,Hkv,D", [(4, 2, 64), (4, 1, 128), (3, 3, 64)])
+@pytest.mark.parametrize("parts", [[(1, 2), (0, 2)], [(126, 2), (127, 2), (0, 129), (1, 127)], [(255, 257), (640, 3), (3, 256)],
+                                   [(1000, 300)]])
+def test_portions_against_the_cache_match_fp64(Hq, Hkv, D, parts):
+    """Gathered keys and the flash kernel with split weights: bf16 rounding of the result (2^-9, doubled) plus what weights of
+    16 bits leave of values up to about five (2^-16 * 5)."""
+    from trainscale_b200.ops import _lib, flash
+    torch.manual_seed(1)
+    dev, bs, kw = "cuda", 16, Hkv * D
+    lens = [s + n for s, n in parts]
+    blocks = [-(-n // bs) for n in lens]
+    kc, vc = (torch.randn(sum(blocks) + 1, bs, Hkv, D, device=dev, dtype=torch.bfloat16) for _ in range(2))
+    kc[-1] = vc[-1] = float("nan")              # a block that nobody holds must not be read
+    order, table = torch.randperm(sum(blocks)), torch.full((len(parts), max(blocks)), sum(blocks), dtype=torch.int32)
+    for i, part in enumerate(order.split(blocks)):
+        table[i, :blocks[i]] = part
+        tail = lens[i] % bs
+        if tail:
+            kc[part[-1], tail:] = vc[part[-1], tail:] = float("nan")
+    table = table.to(dev)
+    rows = [-(-n // 128) * 128 for n in lens]
+    i32 = dict(dtype=torch.int32, device=dev)
+    starts, lens_d = torch.tensor([sum(rows[:i]) for i in range(len(rows))], **i32), torch.tensor(lens, **i32)
+    cu = [3]                                     # three rows of others come first
+    for _, n in parts:
+        cu.append(cu[-1] + n)
+    q = torch.randn(cu[-1], Hq * D + 2 * kw, device=dev, dtype=torch.bfloat16)
+    out = torch.full((cu[-1], Hq * D), 7.0, device=dev, dtype=torch.bfloat16)
+    kv = torch.full((sum(rows), 2 * kw), float("nan"), device=dev, dtype=torch.bfloat16)
+    lib = _lib.load("decode")
+    _lib.check(lib.ts_kv_gather(_lib.ptr(kc), _lib.ptr(vc), _lib.ptr(table), table.shape[1], _lib.ptr(starts), _lib.ptr(lens_d),
+                                len(parts), max(lens), bs, kw, _lib.ptr(kv), _lib.stream_ptr()), "ts_kv_gather")
+    flash.flash_portions(q, kv[:, :kw], kv[:, kw:], out, Hq, Hkv, D, torch.tensor(cu, **i32), starts, lens_d,
+                         max(n for _, n in parts), 1 / math.sqrt(D))
+    torch.cuda.synchronize()
+    _lib.raise_on_any_device_error()
+    assert (out[:3] == 7.0).all()
+    for i, (s, n) in enumerate(parts):
+        k, v = (c[table[i, :blocks[i]].long()].reshape(-1, Hkv, D)[:lens[i]].double().repeat_interleave(Hq // Hkv, 1) for c in (kc, vc))
+        sc = torch.einsum("qhd,khd->hqk", q[cu[i]:cu[i + 1], :Hq * D].double().view(n, Hq, D), k) / math.sqrt(D)
+        hidden = torch.arange(lens[i], device=dev) > torch.arange(s, s + n, device=dev).unsqueeze(1)
+        ref = torch.einsum("hqk,khd->qhd", torch.softmax(sc.masked_fill(hidden, float("-inf")), -1), v).reshape(n, -1)
+        err = (out[cu[i]:cu[i + 1]].double() - ref).abs()
+        assert (err <= 2.0 ** -8 * ref.abs() + 2.0 ** -16 * 5).all(), float(err.max())
+
+
+def test_mixed_steps_give_the_logits_of_the_whole_sequence():
+    """Decoding rows beside first and further portions of prompts in one step; groups of sequences that are gathered apart."""
+    from trainscale_b200.inference import engine as E
+    from trainscale_b200.inference.batch import StepEntry
+    from trainscale_b200.models.llama import LlamaConfig, build_model
+    cfg = LlamaConfig(vocab_size=300, hidden_size=256, intermediate_size=512, num_hidden_layers=2,
+                      num_attention_heads=4, num_key_value_heads=2, head_dim=64)
+    model = build_model(cfg, dtype=torch.bfloat16, device="cuda", seed=1)
+    config = E.EngineConfig(model="tiny", cache=E.CacheConfig(block_size=16, num_gpu_blocks=256, max_model_len=1024))
+    core = E.EngineCore(config, model=model)
+    g = torch.Generator().manual_seed(3)
+    ids = {s: torch.randint(0, 300, (n,), generator=g).tolist() for s, n in ((0, 9), (1, 400), (2, 150), (3, 33))}
+    want = {s: model(torch.tensor([t], device="cuda")).logits[0].float().detach() for s, t in ids.items()}
+    limit, E.GATHER_ROWS = E.GATHER_ROWS, 256
+    try:
+        at = {s: 0 for s in ids}
+        for step in ([(0, 7), (1, 130)], [(2, 1), (1, 200), (0, 1), (3, 20)], [(3, 13), (2, 149), (1, 70), (0, 1)]):
+            logits = core.execute([StepEntry(s, ids[s][at[s]:at[s] + n]) for s, n in step])
+            for (s, n), row in zip(step, logits):
+                at[s] += n
+                ref = want[s][at[s] - 1]
+                assert (row - ref).norm() <= 0.02 * ref.norm(), (s, at[s])
+    finally:
+        E.GATHER_ROWS = limit

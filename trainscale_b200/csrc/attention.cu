@@ -5,7 +5,9 @@
 //   warp 1        MMA issuer (one thread): S_t = Q_t K^T into TMEM, later O_t += P_t V with P_t read from TMEM
 //   warps 2..5    softmax for tile 0, warps 6..9 for tile 1: one thread per query row (its own TMEM lane), so row
 //                 max / sum need no shuffles; P is written back over S as packed bf16, O is rescaled in TMEM
-//                 only when the running max moved by more than 2^8 (exact: O and the row sum share the stale max)
+//                 only when the running max moved by more than 2^8 (exact: O and the row sum share the stale max).
+//                 `SPLIT` (portions of prompts against a cache): P = high + low bf16 parts, both multiplied with V, which
+//                 leaves 16 bits of every weight; the low part takes the other 64 columns of S
 // While one tile's rows are in softmax the tensor core works on the other tile.
 // Backward is two kernels that recompute S and dP: one owns a K/V tile and accumulates dK, dV over the query
 // tiles of its head group; one owns a Q tile and accumulates dQ over the K/V tiles.  No atomics, deterministic.
@@ -23,6 +25,8 @@ struct AttnParams {
   int Hq, Hkv, group;           // group = Hq / Hkv
   int B, S;                     // uniform batch (ignored when cu_seqlens != nullptr)
   const int* cu_seqlens;        // [B + 1] or nullptr
+  const int* k_starts;          // keys apart from the queries: first key row of every sequence (nullptr: the queries' rows)
+  const int* k_lens;            // and its keys; the queries are its last ones
   int causal;
   float scale_log2;             // softmax scale * log2(e)
   __nv_bfloat16* o;             // [rows][o_stride], head h at column h*D
@@ -73,7 +77,7 @@ struct FwdSmem {
 
 constexpr int FWD_THREADS = 320;
 
-template <int D, bool EXT>   // EXT: sliding window / logit soft-cap code paths compiled in
+template <int D, bool EXT, bool SPLIT>   // EXT: sliding window / logit soft-cap code paths compiled in
 __global__ void __launch_bounds__(FWD_THREADS, 1)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, AttnParams p) {
@@ -101,8 +105,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const int hk = h / p.group;
   int q_start, Lq, k_start, Lk;
   seq_bounds(p, b, q_start, Lq);
-  k_start = q_start;
-  Lk = Lq;
+  k_start = SPLIT ? p.k_starts[b] : q_start;
+  Lk = SPLIT ? p.k_lens[b] : Lq;
   const int n_qblocks = (Lq + 255) / 256;
   if ((int)blockIdx.y >= n_qblocks) return;
   const int qb = n_qblocks - 1 - blockIdx.y;   // heaviest (latest) causal blocks first
@@ -205,6 +209,12 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             for (int kk = 0; kk < 8; ++kk)
               umma_f16_ts(tmem_base + O_COL0 + t * D, tmem_base + t * 128 + kk * 8,
                           make_smem_desc_sw128(va + kk * 2048, 16384, 1024), idesc_o, (i | kk) != 0);
+            if (SPLIT) {
+#pragma unroll
+              for (int kk = 0; kk < 8; ++kk)
+                umma_f16_ts(tmem_base + O_COL0 + t * D, tmem_base + t * 128 + 64 + kk * 8,
+                            make_smem_desc_sw128(va + kk * 2048, 16384, 1024), idesc_o, 1u);
+            }
             if (i == nkv[t] - 1) umma_commit(&o_full[t]);
           }
           if (i + 1 < nkv[t]) {
@@ -288,7 +298,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       float l0 = 0.f, l1 = 0.f;
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        uint32_t pk[16];
+        uint32_t pk[16], low[16];
 #pragma unroll
         for (int j = 0; j < 32; j += 2) {
           const float p0 = fast_ex2(fmaf(__uint_as_float(v[c * 32 + j]), sc, -m_sub));
@@ -296,8 +306,13 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           l0 += p0;
           l1 += p1;
           pk[j >> 1] = pack_bf16x2(p0, p1);
+          if (SPLIT) {
+            const float2 high = unpack_bf16x2(pk[j >> 1]);
+            low[j >> 1] = pack_bf16x2(p0 - high.x, p1 - high.y);
+          }
         }
         tmem_st_32x32b_x16(t_s + c * 16, pk);
+        if (SPLIT) tmem_st_32x32b_x16(t_s + 64 + c * 16, low);
       }
       l += l0 + l1;
       tc_wait_st();
@@ -897,18 +912,18 @@ static int launch_bwd(const CUtensorMap* m, const AttnParams& p, int max_len, cu
   return (int)cudaGetLastError();
 }
 
-template <int D, bool EXT>
+template <int D, bool EXT, bool SPLIT = false>
 static int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnParams& p,
                       int max_len, cudaStream_t st) {
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(flash_fwd_kernel<D, EXT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(flash_fwd_kernel<D, EXT, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          FwdSmem<D>::TOTAL);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
   dim3 grid(p.Hq * p.B, (max_len + 255) / 256, 1);
-  flash_fwd_kernel<D, EXT><<<grid, FWD_THREADS, FwdSmem<D>::TOTAL, st>>>(tq, tk, tv, p);
+  flash_fwd_kernel<D, EXT, SPLIT><<<grid, FWD_THREADS, FwdSmem<D>::TOTAL, st>>>(tq, tk, tv, p);
   return (int)cudaGetLastError();
 }
 
@@ -958,6 +973,28 @@ extern "C" int ts_flash_fwd(const void* q, const void* k, const void* v, void* o
                             int causal, float scale, void* stream) {
   return ts_flash_fwd_ex(q, k, v, o, lse, total_rows, q_stride, k_stride, v_stride, o_stride, q_col0, k_col0, v_col0, Hq,
                          Hkv, D, B, S, cu_seqlens, max_len, causal, scale, 0, 0.f, stream);
+}
+
+// Portions of prompts against keys of a cache: sequence b's queries are rows [cu_q[b], cu_q[b + 1]) of q and the LAST of its
+// k_lens[b] keys, which lie at rows k_starts[b] on of k / v (head g of k at column g * D, of v too); rows up to the next
+// multiple of 128 are read, so they hold finite values.  Causal.  Weights keep 16 bits (SPLIT).
+extern "C" int ts_flash_portions(const void* q, const void* k, const void* v, void* o, long long q_rows, long long k_rows,
+                                 int q_stride, int kv_stride, int o_stride, int Hq, int Hkv, int D, int B, const int* cu_q,
+                                 const int* k_starts, const int* k_lens, int max_q, float scale, void* stream) {
+  if ((D != 64 && D != 128) || Hkv <= 0 || Hq % Hkv != 0 || q_rows <= 0 || k_rows <= 0 || B <= 0 || max_q <= 0) return -10;
+  CUtensorMap tq, tk, tv;
+  int rc = make_tmap_2d(&tq, q, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)q_rows, (uint64_t)Hq * D, (uint64_t)q_stride, 128, 64);
+  if (rc) return rc * 100 - 1;
+  rc = make_tmap_2d(&tk, k, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)k_rows, (uint64_t)Hkv * D, (uint64_t)kv_stride, 128, 64);
+  if (rc) return rc * 100 - 2;
+  rc = make_tmap_2d(&tv, v, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)k_rows, (uint64_t)Hkv * D, (uint64_t)kv_stride, 128, 64);
+  if (rc) return rc * 100 - 3;
+  AttnParams p{};
+  p.Hq = Hq; p.Hkv = Hkv; p.group = Hq / Hkv; p.B = B; p.cu_seqlens = cu_q; p.k_starts = k_starts; p.k_lens = k_lens;
+  p.causal = 1; p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
+  p.o = (__nv_bfloat16*)o; p.o_stride = o_stride; p.total_rows = q_rows;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  return D == 128 ? launch_fwd<128, false, true>(tq, tk, tv, p, max_q, st) : launch_fwd<64, false, true>(tq, tk, tv, p, max_q, st);
 }
 
 extern "C" int ts_attn_delta(const void* o, const void* dout, float* delta, long long total_rows, int Hq, int D,

@@ -29,6 +29,31 @@ __global__ void kv_cache_write_kernel(const __nv_bfloat16* __restrict__ qkv, int
   }
 }
 
+// Cached keys and values of sequences side by side, in key order: rows [starts[s], starts[s] + lens[s]) of out
+// [rows][2 * kv_width], the rows up to the next multiple of 128 zero (attention reads whole tiles of 128 keys).
+// grid (rows of the longest / KV_GATHER_ROWS, sequences); one warp per row.
+constexpr int KV_GATHER_ROWS = 8;
+__global__ void __launch_bounds__(KV_GATHER_ROWS * 32)
+kv_gather_kernel(const __nv_bfloat16* __restrict__ k_cache, const __nv_bfloat16* __restrict__ v_cache,
+                 const int* __restrict__ block_table, int max_blocks, const int* __restrict__ starts,
+                 const int* __restrict__ lens, int block_size, int kv_width, __nv_bfloat16* __restrict__ out) {
+  const int s = blockIdx.y, j = blockIdx.x * KV_GATHER_ROWS + (threadIdx.x >> 5), lane = threadIdx.x & 31, len = lens[s];
+  if (j >= (len + 127) / 128 * 128) return;
+  uint4* dst = reinterpret_cast<uint4*>(out + (static_cast<size_t>(starts[s]) + j) * 2 * kv_width);
+  const int vecs = kv_width >> 3;
+  if (j >= len) {
+    for (int v = lane; v < 2 * vecs; v += 32) dst[v] = make_uint4(0u, 0u, 0u, 0u);
+    return;
+  }
+  const size_t slot = static_cast<size_t>(block_table[static_cast<size_t>(s) * max_blocks + j / block_size]) * block_size + j % block_size;
+  const uint4* ks = reinterpret_cast<const uint4*>(k_cache + slot * kv_width);
+  const uint4* vs = reinterpret_cast<const uint4*>(v_cache + slot * kv_width);
+  for (int v = lane; v < vecs; v += 32) {
+    dst[v] = ks[v];
+    dst[vecs + v] = vs[v];
+  }
+}
+
 constexpr int DEC_WARPS = 8;
 constexpr int DEC_MAX_GROUP = 8;
 
@@ -155,6 +180,18 @@ extern "C" int ts_kv_cache_write(const void* qkv, int row_stride, int k_col0, in
   kv_cache_write_kernel<<<(unsigned)blocks, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       (const __nv_bfloat16*)qkv, row_stride, k_col0, v_col0, (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache,
       slot_mapping, rows, kv_width);
+  return (int)cudaGetLastError();
+}
+
+extern "C" int ts_kv_gather(const void* k_cache, const void* v_cache, const int* block_table, int max_blocks,
+                            const int* starts, const int* lens, int sequences, int max_len, int block_size, int kv_width,
+                            void* out, void* stream) {
+  if (sequences <= 0 || max_len <= 0) return 0;
+  if (kv_width % 8 != 0 || block_size <= 0 || sequences > 65535) return -10;
+  const int rows = (max_len + 127) / 128 * 128;
+  kv_gather_kernel<<<dim3(rows / KV_GATHER_ROWS, sequences), KV_GATHER_ROWS * 32, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+      (const __nv_bfloat16*)k_cache, (const __nv_bfloat16*)v_cache, block_table, max_blocks, starts, lens, block_size, kv_width,
+      (__nv_bfloat16*)out);
   return (int)cudaGetLastError();
 }
 

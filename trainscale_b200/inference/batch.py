@@ -48,6 +48,19 @@ class Portions:
         return max(b - a for a, b in zip(self.offsets[:-1], self.offsets[1:]))
 
 
+@dataclass
+class KeyGroup:
+    """Neighbouring multi-token entries [first, end) whose whole contexts are laid side by side, each from a multiple of 128
+    rows on."""
+    first: int
+    end: int
+    rows: int
+    longest: int                  # keys of the longest context
+    max_q: int
+    cu_q: torch.Tensor            # int32 [end - first + 1]: rows of the batch
+    starts: torch.Tensor          # int32 [end - first]: first key row of every entry
+
+
 class HostBatch:
     """Host side of a step: tokens are appended to the cache, index lists are built.  Single-token entries come first
     (`order` maps batch position -> entry), so that decoding rows and portions of prompts are contiguous."""
@@ -160,6 +173,33 @@ class StepBatch:
                 at.append(at[-1] + n)
             self._contexts["portions"] = Portions(at, torch.tensor(at, dtype=torch.int32).to(self.token_ids.device))
         return self._contexts["portions"]
+
+    @property
+    def longest_single(self) -> int:
+        """Upper bound of the keys that a single-token entry sees."""
+        h = self.host
+        return self.max_len if h is None else max(s + 1 for s in h.starts[:self.n_single])
+
+    def key_groups(self, limit: int) -> list[KeyGroup]:
+        """The multi-token entries in groups of at most `limit` key rows (or of one entry), uploaded once per step."""
+        if "key_groups" not in self._contexts:
+            h = self.host
+            n = len(h.q_lens) - h.n_single
+            keys = [h.starts[h.n_single + i] + h.q_lens[h.n_single + i] for i in range(n)]
+            row, bounds, starts, cu = h.n_single, [], [], [h.n_single]
+            for i in range(n):
+                size = -(-keys[i] // 128) * 128
+                if not bounds or bounds[-1][2] + size > limit:
+                    bounds.append([i, i, 0])
+                starts.append(bounds[-1][2])
+                bounds[-1][1:] = [i + 1, bounds[-1][2] + size]
+                row += h.q_lens[h.n_single + i]
+                cu.append(row)
+            dev = torch.tensor(cu + starts, dtype=torch.int32).to(self.token_ids.device)
+            self._contexts["key_groups"] = [
+                KeyGroup(a, b, rows, max(keys[a:b]), max(h.q_lens[h.n_single + a:h.n_single + b]), dev[a:b + 1],
+                         dev[n + 1 + a:n + 1 + b]) for a, b, rows in bounds]
+        return self._contexts["key_groups"]
 
     def prompt_context(self, mask: KeyMask) -> PromptContext | None:
         """Key rows that the multi-token entries see through `mask` (None: no such entries)."""

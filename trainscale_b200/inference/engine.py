@@ -28,7 +28,7 @@ import torch
 from ..utils.refargs import ANY, reference_kwargs
 
 from ..core.types import Err, Ok, Result
-from ..ops import _lib, activation, attention, gemm, norm, rope
+from ..ops import _lib, activation, attention, flash, gemm, norm, rope
 from .batch import HostBatch, StepBatch, StepEntry
 from .kv_cache import CacheSpec, PagedKVCache
 from .sampling import apply_penalties, sample
@@ -250,6 +250,12 @@ class StreamChunk:
 
 
 # ------------------------------------------------------------------------------------------------ model runner
+MAX_DECODE_GROUP = 8         # query heads per key head that ts_decode_attention takes
+# Keys that are laid side by side at a time for portions of prompts: bounds the copy (0.5 GB with 8 key heads of 128) where
+# many long sequences meet in a step; one longer sequence still goes alone
+GATHER_ROWS = 1 << 17
+
+
 class ModelRunner:
     """Runs a decoder over a flattened token batch with the paged cache.  A model that defines `serve(batch, cache)` brings
     its own layers (models/mezilix.py); for `LlamaForCausalLM` they are here."""
@@ -313,33 +319,23 @@ class ModelRunner:
 
     def _attend(self, layer: int, qkv2d: torch.Tensor, batch: StepBatch) -> torch.Tensor:
         c = self.cfg
-        q_lens, fresh, splits = batch.q_lens, batch.fresh, batch.splits
-        block_table, seq_lens = batch.block_table, batch.seq_lens
+        q_lens, fresh = batch.q_lens, batch.fresh
         Hq, Hkv, D = self.Hq, self.Hkv, c.head_dim
         scale = 1.0 / math.sqrt(D)
         T = qkv2d.shape[0]
         if self.cuda and fresh and D in (64, 128):
             # every sequence starts at position 0: packed-prompt flash attention
-            from ..ops import flash
             o, _ = flash.flash_forward_only(qkv2d.unsqueeze(0), Hq, Hkv, D, True, scale, batch.cu_q, max(q_lens))
             return o.view(T, Hq * D)
-        if self.cuda and all(n == 1 for n in q_lens) and D in (64, 128):
-            lib = _lib.load("decode")
-            n = qkv2d.shape[0]
-            chunk = 512
-            if splits is None:       # (a captured decode passes the split count of its block-table width)
-                splits = max(1, -(-batch.max_len // chunk))
-            out = torch.empty(n, Hq * D, dtype=qkv2d.dtype, device=self.device)
-            po = torch.empty(n, Hq, splits, D, dtype=torch.float32, device=self.device)
-            pl = torch.empty(n, Hq, splits, dtype=torch.float32, device=self.device)
-            rc = lib.ts_decode_attention(_lib.ptr(qkv2d), qkv2d.stride(0), _lib.ptr(self.cache.k[layer]),
-                                         _lib.ptr(self.cache.v[layer]), _lib.ptr(block_table), block_table.shape[1],
-                                         _lib.ptr(seq_lens), _lib.ptr(out), Hq * D, _lib.ptr(po), _lib.ptr(pl), n, Hq,
-                                         Hkv, D, self.cache.block_size, chunk, splits, ctypes.c_float(scale),
-                                         _lib.stream_ptr())
-            _lib.check(rc, "ts_decode_attention")
+        if self.cuda and D in (64, 128) and Hq // Hkv <= MAX_DECODE_GROUP:
+            # rows of single tokens come first; the portions of prompts behind them see keys of earlier steps
+            out = torch.empty(T, Hq * D, dtype=qkv2d.dtype, device=self.device)
+            if batch.n_single:
+                self._attend_rows(layer, qkv2d, batch, out, scale)
+            if batch.n_single < len(q_lens):
+                self._attend_portions(layer, qkv2d, batch, out, scale)
             return out
-        # general path (chunked prefill continuation, CPU): per sequence against the gathered cache
+        # general path (CPU, other head sizes): per sequence against the gathered cache
         outs, off = [], 0
         for sid, n in zip(batch.seq_ids, q_lens):
             q = qkv2d[off:off + n, :Hq * D].view(1, n, Hq, D)
@@ -348,6 +344,35 @@ class ModelRunner:
             outs.append(o.reshape(n, Hq * D))
             off += n
         return torch.cat(outs)
+
+    def _attend_rows(self, layer: int, qkv2d: torch.Tensor, batch: StepBatch, out: torch.Tensor, scale: float) -> None:
+        """out[:n] of the batch's first n rows, single tokens of as many sequences."""
+        n, D, table = batch.n_single, self.cfg.head_dim, batch.block_table
+        chunk = 512
+        # a captured decode passes the split count of its block-table width
+        splits = batch.splits or max(1, -(-batch.longest_single // chunk))
+        po = torch.empty(n, self.Hq, splits, D, dtype=torch.float32, device=self.device)
+        pl = torch.empty(n, self.Hq, splits, dtype=torch.float32, device=self.device)
+        rc = _lib.load("decode").ts_decode_attention(
+            _lib.ptr(qkv2d), qkv2d.stride(0), _lib.ptr(self.cache.k[layer]), _lib.ptr(self.cache.v[layer]), _lib.ptr(table),
+            table.shape[1], _lib.ptr(batch.seq_lens), _lib.ptr(out), out.stride(0), _lib.ptr(po), _lib.ptr(pl), n, self.Hq,
+            self.Hkv, D, self.cache.block_size, chunk, splits, ctypes.c_float(scale), _lib.stream_ptr())
+        _lib.check(rc, "ts_decode_attention")
+
+    def _attend_portions(self, layer: int, qkv2d: torch.Tensor, batch: StepBatch, out: torch.Tensor, scale: float) -> None:
+        """out of the rows behind the single tokens: portions of prompts that continue what earlier steps left in the cache.
+        Their sequences' keys and values are laid side by side in key order, as many sequences at a time as
+        GATHER_ROWS allows, and go through the flash kernel."""
+        n, D, bs = batch.n_single, self.cfg.head_dim, self.cache.block_size
+        kw = self.Hkv * D
+        for g in batch.key_groups(GATHER_ROWS):
+            kv = torch.empty(g.rows, 2 * kw, dtype=qkv2d.dtype, device=self.device)
+            table, lens = batch.block_table[n + g.first:n + g.end], batch.seq_lens[n + g.first:n + g.end]
+            rc = _lib.load("decode").ts_kv_gather(
+                _lib.ptr(self.cache.k[layer]), _lib.ptr(self.cache.v[layer]), _lib.ptr(table), table.shape[1],
+                _lib.ptr(g.starts), _lib.ptr(lens), g.end - g.first, g.longest, bs, kw, _lib.ptr(kv), _lib.stream_ptr())
+            _lib.check(rc, "ts_kv_gather")
+            flash.flash_portions(qkv2d, kv[:, :kw], kv[:, kw:], out, self.Hq, self.Hkv, D, g.cu_q, g.starts, lens, g.max_q, scale)
 
     def _layers(self, batch: StepBatch) -> torch.Tensor:
         """The decoder over a flattened token batch; returns the final-norm hidden state of the wanted rows."""

@@ -102,3 +102,18 @@ def flash_forward_only(qkv: torch.Tensor, n_heads: int, n_kv_heads: int, head_di
     else:
         o, lse = _fwd(q2, n_heads, n_kv_heads, head_dim, B, S, None, S, causal, scale)
     return o.view(B, S, -1), lse
+
+
+def flash_portions(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tensor, n_heads: int, n_kv_heads: int,
+                   head_dim: int, cu_q: torch.Tensor, k_starts: torch.Tensor, k_lens: torch.Tensor, max_q: int,
+                   scale: float) -> None:
+    """Causal attention of portions of sequences against all of their keys, without autograd: queries q[cu_q[b]:cu_q[b + 1],
+    :Hq * D] are the last of the k_lens[b] keys at rows k_starts[b] on of k and v [rows, Hkv * D] (same row stride; rows up to
+    the next multiple of 128 hold finite values); results go to the same rows of `out`.  Offsets and lengths are int32."""
+    if k.stride() != v.stride() or k.shape != v.shape:
+        raise ValueError("keys and values are rows of one layout")
+    rc = _lib.load("attention").ts_flash_portions(
+        _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(out), _ll(q.shape[0]), _ll(k.shape[0]), q.stride(0), k.stride(0),
+        out.stride(0), n_heads, n_kv_heads, head_dim, k_starts.numel(), _lib.ptr(cu_q), _lib.ptr(k_starts), _lib.ptr(k_lens),
+        max_q, _f(scale), _lib.stream_ptr())
+    _lib.check(rc, "ts_flash_portions")
