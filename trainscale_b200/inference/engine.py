@@ -286,7 +286,7 @@ class ModelRunner:
         return x
 
     def _lin(self, li: int, wname: str, w: torch.Tensor, x: torch.Tensor, adapter_ids) -> torch.Tensor:
-        y = gemm.linear(x, w)
+        y = gemm.step_linear(x, w)
         if self.lora is not None and adapter_ids is not None:
             d = self.lora.delta(li, wname, x, adapter_ids)
             if d is not None:
@@ -399,9 +399,11 @@ class ModelRunner:
             if hasattr(mlp, "router"):            # mixture of experts: the block routes by itself
                 x = layer.mlp(h)
             else:
-                x = self._reduce(self._lin(li, "w_down", mlp.w_down,
-                                           activation.glu(self._lin(li, "w_gate_up", mlp.w_gate_up, h, adapter_ids),
-                                                          mlp.act), adapter_ids))
+                if self.lora is not None and adapter_ids is not None:
+                    h = activation.glu(self._lin(li, "w_gate_up", mlp.w_gate_up, h, adapter_ids), mlp.act)
+                else:
+                    h = gemm.step_glu(h, mlp.w_gate_up, mlp.act)
+                x = self._reduce(self._lin(li, "w_down", mlp.w_down, h, adapter_ids))
         x, _ = m.norm(x, res)
         return x[batch.out_rows]
 
@@ -469,7 +471,7 @@ class ModelRunner:
               "copied": torch.cuda.Event()}
 
         def body():
-            return self.model.logits(self._layers(batch)).float()
+            return self.logits(self._layers(batch))
 
         side = torch.cuda.Stream(device=dev)
         side.wait_stream(torch.cuda.current_stream())
@@ -485,7 +487,11 @@ class ModelRunner:
 
     @torch.no_grad()
     def logits(self, hidden: torch.Tensor) -> torch.Tensor:
-        return self.model.logits(hidden).float()
+        """fp32 logits of hidden states [n, H]."""
+        if self.own_layers or self.tp is not None or not self.cuda:
+            return self.model.logits(hidden).float()
+        z, cap = gemm.step_linear(hidden, self.model.head_weight, torch.float32), self.cfg.final_logit_softcap
+        return cap * torch.tanh(z / cap) if cap and cap > 0 else z
 
 
 # ------------------------------------------------------------------------------------------------ scheduler / engine core

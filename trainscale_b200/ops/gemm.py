@@ -11,7 +11,7 @@ import ctypes
 
 import torch
 
-from . import _lib
+from . import _lib, activation
 
 _c = ctypes
 
@@ -205,6 +205,47 @@ class _SplitLinearCPU(torch.autograd.Function):
             WgradQueue._active.push(dy2, x, w)
             return dx, None
         return dx, (dy2.t() @ x.reshape(-1, x.shape[-1])).to(w.dtype)
+
+
+def _streamed(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether weight tiles (csrc/rows_gemm.cu) beat 128-row token tiles.  Measured in us, streamed / token tiles, weights not in
+    L2.  Up to 32 rows always: 8 rows 7.6 / 11.5 (3072 x 2048), 83 / 108 (128256 x 2048); 32 rows 42 / 46 (28672 x 4096).  Up to
+    128 where token tiles are too few for the GPU: 128 rows 17.0 / 31.8 (2048 x 8192), 18.2 / 20.3 (6144 x 4096), but
+    20.9 / 15.6 (16384 x 2048).  Beyond, every 128 rows read the weights again (from L2), which pays for a deep reduction:
+    256 rows 18.9 / 31.7 (2048 x 8192), but 23.7 / 20.2 (6144 x 4096)."""
+    if not (x.is_cuda and x.dtype == w.dtype == torch.bfloat16 and x.dim() == 2 and x.shape[0] > 0
+            and all(t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (x, w))):
+        return False
+    M, (N, K) = x.shape[0], w.shape
+    return M <= 32 or N <= 12288 and (M <= 128 or M <= 256 and K >= 3 * N)
+
+
+def _stream_rows(x: torch.Tensor, w: torch.Tensor, cols: int, out_dtype: torch.dtype, glu: int) -> torch.Tensor:
+    out = torch.empty(x.shape[0], cols, dtype=out_dtype, device=x.device)
+    rc = _lib.load("rows_gemm").ts_rows_gemm(
+        _lib.ptr(x), _lib.ptr(w), _lib.ptr(out), x.shape[0], cols, x.shape[1], _c.c_longlong(x.stride(0)),
+        _c.c_longlong(w.stride(0)), _c.c_longlong(cols), int(out_dtype == torch.float32), glu, _lib.stream_ptr())
+    _lib.check(rc, "ts_rows_gemm")
+    return out
+
+
+@torch.no_grad()
+def step_linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = None) -> torch.Tensor:
+    """x [M, K] @ w [N, K]^T of a serving step, optionally with an fp32 result."""
+    if _streamed(x, w):
+        return _stream_rows(x, w, w.shape[0], out_dtype or x.dtype, -1)
+    if out_dtype is not None and x.is_cuda and x.dtype == w.dtype == torch.bfloat16 and x.numel():
+        return matmul_nt(x, w, out_dtype=out_dtype).view(*x.shape[:-1], w.shape[0])
+    y = linear(x, w)
+    return y if out_dtype is None else y.to(out_dtype)
+
+
+@torch.no_grad()
+def step_glu(x: torch.Tensor, w: torch.Tensor, act: str) -> torch.Tensor:
+    """act(x @ gate^T) * (x @ up^T) of a serving step; w [2 I, K] = gate | up."""
+    if _streamed(x, w) and w.shape[0] % 2 == 0:
+        return _stream_rows(x, w, w.shape[0] // 2, x.dtype, activation._ACT[act])
+    return activation.glu(linear(x, w), act)
 
 
 def few_rows(M: int, N: int, K: int) -> bool:
