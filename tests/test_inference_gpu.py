@@ -175,3 +175,41 @@ def test_mixed_steps_give_the_logits_of_the_whole_sequence():
                 assert (row - ref).norm() <= 0.02 * ref.norm(), (s, at[s])
     finally:
         E.GATHER_ROWS = limit
+
+
+# (lengths, splits, least chunk): tiles of 16 keys and their neighbours, shares that are empty, cluster merge and workspace merge
+@pytest.mark.parametrize("Hq,Hkv,D,bs", [(8, 2, 64, 16), (3, 3, 128, 16), (16, 2, 128, 32), (6, 2, 64, 24)])
+@pytest.mark.parametrize("lens,splits,chunk", [([1, 15, 16, 17], 1, 16), ([1, 130, 127, 33], 3, 16), ([700, 1, 64, 1030], 8, 16),
+                                               ([700, 2000, 5, 65], 12, 16), ([512, 513, 100, 1], 2, 512)])
+def test_decode_attention_matches_fp64(Hq, Hkv, D, bs, lens, splits, chunk):
+    """Rounding of the result to bf16 (2^-9, doubled) and weights of 16 bits times values up to about five."""
+    import ctypes
+    from trainscale_b200.ops import _lib
+    torch.manual_seed(2)
+    dev, n, kw = "cuda", len(lens), Hkv * D
+    blocks = [-(-k // bs) for k in lens]
+    kc, vc = (torch.randn(sum(blocks) + 1, bs, Hkv, D, device=dev, dtype=torch.bfloat16) for _ in range(2))
+    kc[-1] = vc[-1] = float("nan")              # neither foreign blocks nor the rest of the last one may count
+    table = torch.full((n, max(blocks) + 1), sum(blocks), dtype=torch.int32)
+    for i, part in enumerate(torch.randperm(sum(blocks)).split(blocks)):
+        table[i, :blocks[i]] = part
+        if lens[i] % bs:
+            kc[part[-1], lens[i] % bs:] = vc[part[-1], lens[i] % bs:] = float("nan")
+    table = table.to(dev)
+    q = torch.randn(n, Hq * D + 2 * kw, device=dev, dtype=torch.bfloat16)
+    out = torch.empty(n, Hq * D, device=dev, dtype=torch.bfloat16)
+    po = torch.empty(n, Hq, splits, D, device=dev) if splits > 8 else None
+    pl = torch.empty(n, Hq, splits, device=dev) if splits > 8 else None
+    lib = _lib.load("decode")
+    rc = lib.ts_decode_attention(_lib.ptr(q), q.stride(0), _lib.ptr(kc), _lib.ptr(vc), _lib.ptr(table), table.shape[1],
+                                 _lib.ptr(torch.tensor(lens, dtype=torch.int32, device=dev)), _lib.ptr(out), Hq * D,
+                                 _lib.ptr(po), _lib.ptr(pl), n, Hq, Hkv, D, bs, chunk, splits,
+                                 ctypes.c_float(1 / math.sqrt(D)), _lib.stream_ptr())
+    assert rc == 0
+    torch.cuda.synchronize()
+    for i, m in enumerate(lens):
+        k, v = (c[table[i, :blocks[i]].long()].reshape(-1, Hkv, D)[:m].double().repeat_interleave(Hq // Hkv, 1) for c in (kc, vc))
+        w = torch.softmax(torch.einsum("hd,khd->hk", q[i, :Hq * D].double().view(Hq, D), k) / math.sqrt(D), -1)
+        ref = torch.einsum("hk,khd->hd", w, v).reshape(-1)
+        err = (out[i].double() - ref).abs()
+        assert (err <= 2.0 ** -8 * ref.abs() + 2.0 ** -15 * 5).all(), (i, float(err.max()))

@@ -504,6 +504,20 @@ __device__ __forceinline__ void st_shared_cluster(float* p, uint32_t cta, float 
       "r"(cta), "f"(v)
       : "memory");
 }
+// read from the same smem offset in CTA `cta` of this cluster
+__device__ __forceinline__ float ld_shared_cluster(const float* p, uint32_t cta) {
+  float v;
+  asm volatile(
+      "{\n\t"
+      ".reg .b32 ra;\n\t"
+      "mapa.shared::cluster.u32 ra, %1, %2;\n\t"
+      "ld.shared::cluster.f32 %0, [ra];\n\t"
+      "}\n"
+      : "=f"(v)
+      : "r"(smem_u32(p)), "r"(cta)
+      : "memory");
+  return v;
+}
 // arrive on the barrier at the same smem offset in CTA `cta` of this cluster
 __device__ __forceinline__ void mbar_arrive_cluster(uint64_t* bar, uint32_t cta) {
   asm volatile(

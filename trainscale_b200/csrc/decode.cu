@@ -1,8 +1,6 @@
 // Inference kernels: paged KV-cache writes and single-token (decode) attention over a paged cache with split-KV.
 //
-// Decode attention is bandwidth-bound (every K/V byte of the sequence is read once per step), so it runs on CUDA
-// cores with 16-byte loads: one warp per cached token, lanes split the head dimension, the q heads of a GQA group
-// share each K/V row.  Long sequences are split over CTAs (gridDim.z) and merged by LSE.
+// Decode attention reads every K/V byte of a sequence once per step; the q heads of a GQA group share each K/V row.
 // Serves the role of the vLLM paged-attention kernels configured in the reference
 // (data_pipeline/trainer/inference.py:786-921) and of data_pipeline/trainer/kernels/flex_attention.py:1032.
 #include "common.cuh"
@@ -54,99 +52,237 @@ kv_gather_kernel(const __nv_bfloat16* __restrict__ k_cache, const __nv_bfloat16*
   }
 }
 
-constexpr int DEC_WARPS = 8;
+constexpr int DEC_WARPS = 4;
 constexpr int DEC_MAX_GROUP = 8;
+constexpr int DEC_MAX_CLUSTER = 8;
 
-// grid (num_seqs, Hkv, splits). Each CTA covers tokens [split*chunk, (split+1)*chunk) of one sequence for one kv head
-// and all `group` q heads that share it. Writes partial out [seq][Hq][split][D] fp32 + lse [seq][Hq][split].
-template <int D>
+__device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                               uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// grid (splits, Hkv, sequences).  A CTA takes an even share of one sequence's keys for one kv head and all query heads that share
+// it.  Memory should bound this; scalar code for four heads of 128 spends 5 - 10 times as many issue slots per key as the loads
+// leave (shuffles of the dot products, conversions), so both products are warp MMAs whose operands come straight from global
+// memory as 16-byte vectors:
+//   S = Q K^T  rows are heads; a lane's eight consecutive dimensions feed two reduction steps (Q in the same order)
+//   O += P V   a lane has the same dimensions of four keys, two keys of one dimension are one operand word; P comes from S in
+//              registers.  The heads use eight of the sixteen rows, so the rows 8 - 15 hold what the bf16 weights of rows 0 - 7
+//              leave over: weights keep 16 bits at no cost
+// Every warp walks its own 16-key tiles with a softmax state of its own; states meet in shared memory, then over the splits: up
+// to DEC_MAX_CLUSTER in distributed shared memory, more through partial results [seq][Hq][split][D] fp32 and lse
+// [seq][Hq][split] for decode_merge_kernel.
+// One warp per key with shuffled dot products / this (32 query heads of 8 kv heads, us; at the copy bandwidth): 64 sequences of
+// 300 keys of 64 75 / 14.5 (6.1), of 2000 keys of 128 571 / 101 (81), 4 of 10000 keys of 128 249 / 37 (25), 1 of 100 of 64 16 / 5.
+template <int D, bool CLUSTER>
 __global__ void __launch_bounds__(DEC_WARPS * 32)
 decode_attention_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, const __nv_bfloat16* __restrict__ k_cache,
                         const __nv_bfloat16* __restrict__ v_cache, const int* __restrict__ block_table,
-                        int max_blocks, const int* __restrict__ seq_lens, float* __restrict__ part_out,
-                        float* __restrict__ part_lse, int Hq, int Hkv, int block_size, int chunk, int splits,
-                        float scale) {
-  constexpr int EPL = D / 32;   // elements per lane
-  const int seq = blockIdx.x, hk = blockIdx.y, split = blockIdx.z;
+                        int max_blocks, const int* __restrict__ seq_lens, __nv_bfloat16* __restrict__ out, int out_stride,
+                        float* __restrict__ part_out, float* __restrict__ part_lse, int Hq, int Hkv, int block_size,
+                        int chunk, int splits, float scale_log2) {
+  constexpr int KT = D == 64 ? 2 : 1;      // 16-key tiles in flight: 8 KB of keys and values per warp
+  constexpr int NK = D / 32, NV = D / 64;
+  const int split = blockIdx.x, hk = blockIdx.y, seq = blockIdx.z;
   const int group = Hq / Hkv;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
   const int len = seq_lens[seq];
-  const int t0 = split * chunk, t1 = min(len, t0 + chunk);
-  __shared__ float s_acc[DEC_WARPS][DEC_MAX_GROUP][D];
+  const int share = (max(chunk, (len + splits - 1) / splits) + 15) & ~15;
+  const int t0 = split * share, t1 = min(len, t0 + share);
+  __shared__ __align__(16) float s_acc[DEC_WARPS][DEC_MAX_GROUP][D];
   __shared__ float s_m[DEC_WARPS][DEC_MAX_GROUP], s_l[DEC_WARPS][DEC_MAX_GROUP];
+  __shared__ __align__(16) float c_acc[DEC_MAX_GROUP][D];      // the CTA's result, not normalised
+  __shared__ float c_m[DEC_MAX_GROUP], c_l[DEC_MAX_GROUP];
 
-  float qv[DEC_MAX_GROUP][EPL];
+  uint4 qv[NK];
 #pragma unroll
-  for (int g = 0; g < DEC_MAX_GROUP; ++g) {
-    if (g < group) {
-      const __nv_bfloat16* qp = q + static_cast<size_t>(seq) * q_stride + (hk * group + g) * D + lane * EPL;
+  for (int i = 0; i < NK; ++i)
+    qv[i] = gid < group ? *reinterpret_cast<const uint4*>(q + static_cast<size_t>(seq) * q_stride + (hk * group + gid) * D + i * 32 + tig * 8)
+                        : make_uint4(0u, 0u, 0u, 0u);
+  float m = -INFINITY, l = 0.f;            // of head gid; l of this lane's keys
+  float acc[NV * 8][4];                    // [n]: columns 2 tig, 2 tig + 1 <-> dimensions 64 (n / 8) + 8 column + n % 8
 #pragma unroll
-      for (int e = 0; e < EPL; ++e) qv[g][e] = __bfloat162float(qp[e]) * scale;
-    }
-  }
-  float m[DEC_MAX_GROUP], l[DEC_MAX_GROUP], acc[DEC_MAX_GROUP][EPL];
+  for (int n = 0; n < NV * 8; ++n)
 #pragma unroll
-  for (int g = 0; g < DEC_MAX_GROUP; ++g) {
-    m[g] = -INFINITY;
-    l[g] = 0.f;
-#pragma unroll
-    for (int e = 0; e < EPL; ++e) acc[g][e] = 0.f;
-  }
+    for (int e = 0; e < 4; ++e) acc[n][e] = 0.f;
   const int kv_width = Hkv * D;
-  for (int t = t0 + warp; t < t1; t += DEC_WARPS) {
-    const int blk = block_table[seq * max_blocks + t / block_size];
-    const size_t slot = static_cast<size_t>(blk) * block_size + (t % block_size);
-    const __nv_bfloat16* kp = k_cache + slot * kv_width + hk * D + lane * EPL;
-    const __nv_bfloat16* vp = v_cache + slot * kv_width + hk * D + lane * EPL;
-    float kf[EPL], vf[EPL];
+  const int* table = block_table + static_cast<size_t>(seq) * max_blocks;
+  // first cache row of a 16-key tile whose keys lie in one block; one past the end repeats the last one, masked below.  The
+  // block table is read two steps ahead and the next step's lines are asked into L2, so that a step waits for L2 only
+  const bool whole = (block_size & 15) == 0;
+  constexpr int STRIDE = DEC_WARPS * 16 * KT;
+  auto tile_base = [&](int t) { return min(t, (t1 - 1) & ~15); };
+  auto tile_first = [&](int t) {
+    const int base = tile_base(t);
+    return whole ? table[base / block_size] * static_cast<long long>(block_size) + base % block_size : 0ll;
+  };
+  long long cur[KT], next[KT], later[KT];
+  if (t0 + warp * 16 * KT < t1) {
 #pragma unroll
-    for (int e = 0; e < EPL; ++e) {
-      kf[e] = __bfloat162float(kp[e]);
-      vf[e] = __bfloat162float(vp[e]);
-    }
-#pragma unroll
-    for (int g = 0; g < DEC_MAX_GROUP; ++g) {
-      if (g < group) {
-        float s = 0.f;
-#pragma unroll
-        for (int e = 0; e < EPL; ++e) s += qv[g][e] * kf[e];
-        s = warp_sum(s);
-        const float mn = fmaxf(m[g], s);
-        const float a = __expf(m[g] - mn), p = __expf(s - mn);
-        l[g] = l[g] * a + p;
-#pragma unroll
-        for (int e = 0; e < EPL; ++e) acc[g][e] = acc[g][e] * a + p * vf[e];
-        m[g] = mn;
-      }
+    for (int x = 0; x < KT; ++x) {
+      cur[x] = tile_first(t0 + (warp * KT + x) * 16);
+      next[x] = tile_first(t0 + (warp * KT + x) * 16 + STRIDE);
     }
   }
-  // merge the warps of this CTA
+  for (int t = t0 + warp * 16 * KT; t < t1; t += STRIDE) {
 #pragma unroll
-  for (int g = 0; g < DEC_MAX_GROUP; ++g) {
-    if (g < group) {
-      if (lane == 0) {
-        s_m[warp][g] = m[g];
-        s_l[warp][g] = l[g];
+    for (int x = 0; x < KT; ++x) later[x] = tile_first(t + 2 * STRIDE + x * 16);
+    uint4 kr[KT][2][NK], vr[KT][4][NV];
+#pragma unroll
+    for (int x = 0; x < KT; ++x) {
+      const int base = tile_base(t + x * 16);
+      auto row = [&](int j) {
+        const int key = min(base + j, t1 - 1);
+        const size_t slot = whole ? cur[x] + (key - base) : static_cast<size_t>(table[key / block_size]) * block_size + key % block_size;
+        return slot * kv_width + hk * D;
+      };
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        const __nv_bfloat16* p = k_cache + row(n * 8 + gid) + tig * 8;
+#pragma unroll
+        for (int i = 0; i < NK; ++i) kr[x][n][i] = *reinterpret_cast<const uint4*>(p + i * 32);
       }
 #pragma unroll
-      for (int e = 0; e < EPL; ++e) s_acc[warp][g][lane * EPL + e] = acc[g][e];
+      for (int j = 0; j < 4; ++j) {
+        const __nv_bfloat16* p = v_cache + row((j >> 1) * 8 + tig * 2 + (j & 1)) + gid * 8;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) vr[x][j][i] = *reinterpret_cast<const uint4*>(p + i * 64);
+      }
+    }
+    if (whole) {
+      // 32 lines of keys and of values: rows of one 128-byte line each (D = 64, two tiles) or of two (D = 128)
+      const int x = KT == 2 ? lane >> 4 : 0, j = KT == 2 ? lane & 15 : lane >> 1;
+      const int key = min(tile_base(t + STRIDE + x * 16) + j, t1 - 1);
+      const size_t at = (next[x] + (key - tile_base(t + STRIDE + x * 16))) * kv_width + hk * D + (KT == 2 ? 0 : (lane & 1) * 64);
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(k_cache + at));
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(v_cache + at));
+    }
+#pragma unroll
+    for (int x = 0; x < KT; ++x) {
+      float s[2][4];
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[n][e] = 0.f;
+#pragma unroll
+        for (int i = 0; i < NK; ++i) {
+          mma_bf16_16816(s[n], qv[i].x, 0u, qv[i].y, 0u, kr[x][n][i].x, kr[x][n][i].y);
+          mma_bf16_16816(s[n], qv[i].z, 0u, qv[i].w, 0u, kr[x][n][i].z, kr[x][n][i].w);
+        }
+      }
+      const int k0 = t + x * 16 + tig * 2;
+      float mn = m;
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          s[n][e] = k0 + n * 8 + e < t1 ? s[n][e] * scale_log2 : -INFINITY;
+          mn = fmaxf(mn, s[n][e]);
+        }
+      mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 1));
+      mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 2));
+      const float sub = mn == -INFINITY ? 0.f : mn;
+      if (__any_sync(0xffffffffu, mn > m)) {
+        const float a = fast_ex2(m - sub);
+        l *= a;
+#pragma unroll
+        for (int n = 0; n < NV * 8; ++n)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[n][e] *= a;
+        m = mn;
+      }
+      uint32_t high[2], low[2];
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        const float p0 = fast_ex2(s[n][0] - sub), p1 = fast_ex2(s[n][1] - sub);
+        l += p0 + p1;
+        high[n] = pack_bf16x2(p0, p1);
+        const float2 h = unpack_bf16x2(high[n]);
+        low[n] = pack_bf16x2(p0 - h.x, p1 - h.y);
+      }
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        const uint32_t v[4][4] = {{vr[x][0][i].x, vr[x][0][i].y, vr[x][0][i].z, vr[x][0][i].w},
+                                  {vr[x][1][i].x, vr[x][1][i].y, vr[x][1][i].z, vr[x][1][i].w},
+                                  {vr[x][2][i].x, vr[x][2][i].y, vr[x][2][i].z, vr[x][2][i].w},
+                                  {vr[x][3][i].x, vr[x][3][i].y, vr[x][3][i].z, vr[x][3][i].w}};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          mma_bf16_16816(acc[i * 8 + 2 * e], high[0], low[0], high[1], low[1], __byte_perm(v[0][e], v[1][e], 0x5410),
+                         __byte_perm(v[2][e], v[3][e], 0x5410));
+          mma_bf16_16816(acc[i * 8 + 2 * e + 1], high[0], low[0], high[1], low[1], __byte_perm(v[0][e], v[1][e], 0x7632),
+                         __byte_perm(v[2][e], v[3][e], 0x7632));
+        }
+      }
+    }
+#pragma unroll
+    for (int x = 0; x < KT; ++x) {
+      cur[x] = next[x];
+      next[x] = later[x];
     }
   }
+  l += __shfl_xor_sync(0xffffffffu, l, 1);
+  l += __shfl_xor_sync(0xffffffffu, l, 2);
+  if (tig == 0) {
+    s_m[warp][gid] = m;
+    s_l[warp][gid] = l;
+  }
+#pragma unroll
+  for (int i = 0; i < NV; ++i)
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      float* dst = &s_acc[warp][gid][i * 64 + (2 * tig + c) * 8];
+#pragma unroll
+      for (int n = 0; n < 8; n += 4)
+        *reinterpret_cast<float4*>(dst + n) =
+            make_float4(acc[i * 8 + n][c] + acc[i * 8 + n][c + 2], acc[i * 8 + n + 1][c] + acc[i * 8 + n + 1][c + 2],
+                        acc[i * 8 + n + 2][c] + acc[i * 8 + n + 2][c + 2], acc[i * 8 + n + 3][c] + acc[i * 8 + n + 3][c + 2]);
+    }
   __syncthreads();
   for (int idx = threadIdx.x; idx < group * D; idx += blockDim.x) {
-    const int g = idx / D, d = idx - g * D;
+    const int g = idx / D, d = idx % D;
     float mm = -INFINITY;
+#pragma unroll
     for (int w = 0; w < DEC_WARPS; ++w) mm = fmaxf(mm, s_m[w][g]);
+    const float sub = mm == -INFINITY ? 0.f : mm;
     float ll = 0.f, o = 0.f;
+#pragma unroll
     for (int w = 0; w < DEC_WARPS; ++w) {
-      const float a = (s_m[w][g] == -INFINITY) ? 0.f : __expf(s_m[w][g] - mm);
+      const float a = fast_ex2(s_m[w][g] - sub);
       ll += s_l[w][g] * a;
       o += s_acc[w][g][d] * a;
     }
-    const int h = hk * group + g;
-    const size_t base = (static_cast<size_t>(seq) * Hq + h) * splits + split;
-    part_out[base * D + d] = ll > 0.f ? o / ll : 0.f;
-    if (d == 0) part_lse[base] = ll > 0.f ? mm + __logf(ll) : -INFINITY;
+    if (CLUSTER) {
+      c_acc[g][d] = o;
+      if (d == 0) {
+        c_m[g] = mm;
+        c_l[g] = ll;
+      }
+    } else {
+      const size_t base = (static_cast<size_t>(seq) * Hq + hk * group + g) * splits + split;
+      part_out[base * D + d] = ll > 0.f ? o / ll : 0.f;
+      if (d == 0) part_lse[base] = ll > 0.f ? mm + log2f(ll) : -INFINITY;
+    }
+  }
+  if (CLUSTER) {
+    if (splits > 1) cluster_sync_all();
+    else __syncthreads();
+    for (int idx = split * (DEC_WARPS * 32) + threadIdx.x; idx < group * D; idx += splits * (DEC_WARPS * 32)) {
+      const int g = idx / D, d = idx % D;
+      float mm = -INFINITY, ll = 0.f, o = 0.f;
+      for (int r = 0; r < splits; ++r) mm = fmaxf(mm, splits > 1 ? ld_shared_cluster(&c_m[g], r) : c_m[g]);
+      const float sub = mm == -INFINITY ? 0.f : mm;
+      for (int r = 0; r < splits; ++r) {
+        const float a = fast_ex2((splits > 1 ? ld_shared_cluster(&c_m[g], r) : c_m[g]) - sub);
+        ll += a * (splits > 1 ? ld_shared_cluster(&c_l[g], r) : c_l[g]);
+        o += a * (splits > 1 ? ld_shared_cluster(&c_acc[g][d], r) : c_acc[g][d]);
+      }
+      out[static_cast<size_t>(seq) * out_stride + (hk * group + g) * D + d] = __float2bfloat16(ll > 0.f ? o / ll : 0.f);
+    }
+    if (splits > 1) cluster_sync_all();            // nobody leaves while a peer may still read its result
   }
 }
 
@@ -159,7 +295,7 @@ __global__ void decode_merge_kernel(const float* __restrict__ part_out, const fl
   for (int s = 0; s < splits; ++s) mm = fmaxf(mm, part_lse[base + s]);
   float den = 0.f, o = 0.f;
   for (int s = 0; s < splits; ++s) {
-    const float w = (part_lse[base + s] == -INFINITY) ? 0.f : __expf(part_lse[base + s] - mm);
+    const float w = (part_lse[base + s] == -INFINITY) ? 0.f : fast_ex2(part_lse[base + s] - mm);
     den += w;
     o += w * part_out[(base + s) * D + d];
   }
@@ -195,26 +331,66 @@ extern "C" int ts_kv_gather(const void* k_cache, const void* v_cache, const int*
   return (int)cudaGetLastError();
 }
 
-// part_out: fp32 [num_seqs][Hq][splits][D], part_lse: fp32 [num_seqs][Hq][splits] (caller-provided workspace);
-// splits = ceil(max_len / chunk).
+namespace ts {
+
+template <int D, bool CLUSTER>
+static int launch_decode(const void* q, int q_stride, const void* k_cache, const void* v_cache, const int* block_table,
+                         int max_blocks, const int* seq_lens, void* out, int out_stride, float* part_out, float* part_lse,
+                         int num_seqs, int Hq, int Hkv, int block_size, int chunk, int splits, float scale_log2, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(splits, Hkv, num_seqs);
+  cfg.blockDim = dim3(DEC_WARPS * 32);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = CLUSTER ? splits : 1;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&cfg, decode_attention_kernel<D, CLUSTER>, (const __nv_bfloat16*)q, q_stride,
+                                 (const __nv_bfloat16*)k_cache, (const __nv_bfloat16*)v_cache, block_table, max_blocks, seq_lens,
+                                 (__nv_bfloat16*)out, out_stride, part_out, part_lse, Hq, Hkv, block_size, chunk, splits,
+                                 scale_log2);
+}
+
+}  // namespace ts
+
+// Shares of a sequence's keys: 256 CTAs in all, at least 128 keys each.  Up to eight are merged inside the kernel; more (long
+// sequences, few heads) cost a second launch and are taken where the eight would have more than 512 keys each.  Measured (us by
+// splits, 8 kv heads): 1 x 10000 keys of 128 27 (8) / 16 (32), 4 x 10000 59 (4) / 37 (8) / 43 (16), 64 x 300 keys of 64
+// 14.5 (1) / 20 (2), 1 x 1000 13 (1) / 6 (8).
+extern "C" int ts_decode_splits(int num_seqs, int Hkv, int max_len) {
+  const long long ctas = static_cast<long long>(num_seqs) * Hkv;
+  int want = ctas > 0 ? static_cast<int>((256 + ctas - 1) / ctas) : 1;
+  const int most = max_len / 128;
+  if (want > most) want = most;
+  if (want > DEC_MAX_CLUSTER && max_len <= DEC_MAX_CLUSTER * 512) want = DEC_MAX_CLUSTER;
+  return want < 1 ? 1 : want;
+}
+
+// chunk: least number of keys of a split (multiples of 16 keep whole cache blocks together); splits * chunk may exceed the keys.
+// splits > 8 (DEC_MAX_CLUSTER): part_out fp32 [num_seqs][Hq][splits][D], part_lse fp32 [num_seqs][Hq][splits] (caller-provided
+// workspace); else they are not used.
 extern "C" int ts_decode_attention(const void* q, int q_stride, const void* k_cache, const void* v_cache,
                                    const int* block_table, int max_blocks, const int* seq_lens, void* out,
                                    int out_stride, float* part_out, float* part_lse, int num_seqs, int Hq, int Hkv,
                                    int D, int block_size, int chunk, int splits, float scale, void* stream) {
   if (num_seqs <= 0) return 0;
-  if (Hq % Hkv != 0 || Hq / Hkv > DEC_MAX_GROUP || (D != 64 && D != 128)) return -10;
+  if (Hkv <= 0 || Hq % Hkv != 0 || Hq / Hkv > DEC_MAX_GROUP || (D != 64 && D != 128) || splits <= 0 || num_seqs > 65535 ||
+      Hkv > 65535)
+    return -10;
+  if (q_stride % 8 || (reinterpret_cast<uintptr_t>(q) & 15u)) return -11;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  dim3 grid(num_seqs, Hkv, splits);
-  if (D == 128) {
-    decode_attention_kernel<128><<<grid, DEC_WARPS * 32, 0, st>>>(
-        (const __nv_bfloat16*)q, q_stride, (const __nv_bfloat16*)k_cache, (const __nv_bfloat16*)v_cache, block_table,
-        max_blocks, seq_lens, part_out, part_lse, Hq, Hkv, block_size, chunk, splits, scale);
+  const float sl = scale * 1.4426950408889634f;
+  const bool cluster = splits <= DEC_MAX_CLUSTER;
+  auto launch = D == 128 ? (cluster ? launch_decode<128, true> : launch_decode<128, false>)
+                         : (cluster ? launch_decode<64, true> : launch_decode<64, false>);
+  const int rc = launch(q, q_stride, k_cache, v_cache, block_table, max_blocks, seq_lens, out, out_stride, part_out, part_lse,
+                        num_seqs, Hq, Hkv, block_size, chunk, splits, sl, st);
+  if (rc || cluster) return rc;
+  if (D == 128)
     decode_merge_kernel<128><<<dim3(num_seqs, Hq), 128, 0, st>>>(part_out, part_lse, (__nv_bfloat16*)out, out_stride, Hq, splits);
-  } else {
-    decode_attention_kernel<64><<<grid, DEC_WARPS * 32, 0, st>>>(
-        (const __nv_bfloat16*)q, q_stride, (const __nv_bfloat16*)k_cache, (const __nv_bfloat16*)v_cache, block_table,
-        max_blocks, seq_lens, part_out, part_lse, Hq, Hkv, block_size, chunk, splits, scale);
+  else
     decode_merge_kernel<64><<<dim3(num_seqs, Hq), 64, 0, st>>>(part_out, part_lse, (__nv_bfloat16*)out, out_stride, Hq, splits);
-  }
   return (int)cudaGetLastError();
 }

@@ -132,7 +132,6 @@ class StepBatch:
     max_len: int                      # upper bound of seq_lens
     fresh: bool                       # every sequence starts at position 0
     adapter_ids: torch.Tensor | None = None
-    splits: int | None = None         # captured decode: split count of the block-table width
     _contexts: dict = field(default_factory=dict)
 
     @property

@@ -251,6 +251,7 @@ class StreamChunk:
 
 # ------------------------------------------------------------------------------------------------ model runner
 MAX_DECODE_GROUP = 8         # query heads per key head that ts_decode_attention takes
+DECODE_CLUSTER = 8           # splits that it merges without a workspace
 # Keys that are laid side by side at a time for portions of prompts: bounds the copy (0.5 GB with 8 key heads of 128) where
 # many long sequences meet in a step; one longer sequence still goes alone
 GATHER_ROWS = 1 << 17
@@ -348,15 +349,16 @@ class ModelRunner:
     def _attend_rows(self, layer: int, qkv2d: torch.Tensor, batch: StepBatch, out: torch.Tensor, scale: float) -> None:
         """out[:n] of the batch's first n rows, single tokens of as many sequences."""
         n, D, table = batch.n_single, self.cfg.head_dim, batch.block_table
-        chunk = 512
-        # a captured decode passes the split count of its block-table width
-        splits = batch.splits or max(1, -(-batch.longest_single // chunk))
-        po = torch.empty(n, self.Hq, splits, D, dtype=torch.float32, device=self.device)
-        pl = torch.empty(n, self.Hq, splits, dtype=torch.float32, device=self.device)
-        rc = _lib.load("decode").ts_decode_attention(
+        lib = _lib.load("decode")
+        splits = lib.ts_decode_splits(n, self.Hkv, batch.longest_single)
+        po = pl = None
+        if splits > DECODE_CLUSTER:
+            po = torch.empty(n, self.Hq, splits, D, dtype=torch.float32, device=self.device)
+            pl = torch.empty(n, self.Hq, splits, dtype=torch.float32, device=self.device)
+        rc = lib.ts_decode_attention(
             _lib.ptr(qkv2d), qkv2d.stride(0), _lib.ptr(self.cache.k[layer]), _lib.ptr(self.cache.v[layer]), _lib.ptr(table),
             table.shape[1], _lib.ptr(batch.seq_lens), _lib.ptr(out), out.stride(0), _lib.ptr(po), _lib.ptr(pl), n, self.Hq,
-            self.Hkv, D, self.cache.block_size, chunk, splits, ctypes.c_float(scale), _lib.stream_ptr())
+            self.Hkv, D, self.cache.block_size, 16, splits, ctypes.c_float(scale), _lib.stream_ptr())
         _lib.check(rc, "ts_decode_attention")
 
     def _attend_portions(self, layer: int, qkv2d: torch.Tensor, batch: StepBatch, out: torch.Tensor, scale: float) -> None:
@@ -465,8 +467,7 @@ class ModelRunner:
         buf = {k: torch.full((n_pad,), pad, dtype=dt, device=dev) for k, (dt, pad) in self._static_fields().items()}
         buf["block_table"] = torch.full((n_pad, width), trash, dtype=torch.int32, device=dev)
         rows = torch.arange(n_pad, dtype=torch.int32, device=dev)
-        batch = StepBatch(None, row_seq=rows, out_rows=rows, n_single=n_pad, max_len=width * bs, fresh=False,
-                          splits=max(1, -(-(width * bs) // 512)), **buf)
+        batch = StepBatch(None, row_seq=rows, out_rows=rows, n_single=n_pad, max_len=width * bs, fresh=False, **buf)
         st = {"batch": batch, "host": {k: torch.empty_like(v, device="cpu").pin_memory() for k, v in buf.items()},
               "copied": torch.cuda.Event()}
 
