@@ -376,53 +376,86 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __n
 }
 
 
+// 32 accumulator columns of the thread's row, scaled, as bf16
+__device__ __forceinline__ void store_rows_32(uint32_t taddr, float scale, __nv_bfloat16* dst, bool valid) {
+  uint32_t v[32];
+  tmem_ld_32x32b_x32(taddr, v);
+  tc_wait_ld();
+  if (!valid) return;
+#pragma unroll
+  for (int x = 0; x < 4; ++x) {
+    uint32_t o[4];
+#pragma unroll
+    for (int y = 0; y < 4; ++y)
+      o[y] = pack_bf16x2(__uint_as_float(v[8 * x + 2 * y]) * scale, __uint_as_float(v[8 * x + 2 * y + 1]) * scale);
+    *reinterpret_cast<uint4*>(dst + x * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+}
+
 // ------------------------------------------------------------------------------------------------
-// backward, kernel 1: dK / dV.  One CTA owns a 128-row K/V tile of one kv head and walks the 64-row query
-// sub-tiles of every query head in its group.  TMEM: two (S^T | dP^T) buffers of 64+64 columns, dV and dK
-// accumulators.  P^T and dS^T are written back over S^T / dP^T as packed bf16 and fed to the MMA from TMEM.
+// backward.  Both kernels work on 128 x 128 blocks of S: an SS product of 128 x 128 takes from shared memory what the tensor core
+// takes in the same time, one of 128 x 64 half as much again.  Bounds per block (D = 128): tensor core 2048 (dK, dV) and 1536 (dQ)
+// cycles, exponentials 1024 cycles of the special-function units, so the products of one block run while the other half of its
+// neighbour is in the compute warps:
+//   dK, dV   dV += P dO and the next block's S   beside   dS = P (dP - delta)
+//            dK += dS Q and the next block's dP  beside   the next block's P = exp2(S - lse)
+//   dQ       dQ += dS K, the next dP, S after it beside   the next block's P and dS (two S buffers)
+// P stays in fp32 registers between its two uses.  Two warpgroups share a row: each has 64 columns of S and dP and writes its
+// bf16 P and dS over the first 32 columns of ITS half, so neither touches columns the other has still to read.
+// 64-wide sub-tiles with P and dS in one phase / this, both kernels, ms (tensor rate over the seven products): S = 8192, 32 / 8
+// heads of 128 1.86 / 1.41 (1360 TFLOP/s), S = 32768 30.5 / 24.9 (1236, power-capped), S = 8192 with heads of 64 2.01 / 1.54 (bound
+// by the exponentials).
+// ------------------------------------------------------------------------------------------------
+constexpr int BWD_THREADS = 320;   // warp 0 TMA, warp 1 MMA, warps 2..5 and 6..9: two compute warpgroups (64 columns each)
+
+// TMEM column of reduction step kk (16 values) of a bf16 operand that the two warpgroups wrote over their halves
+__device__ __forceinline__ uint32_t half_col(int kk) { return (kk >> 2) * 64 + (kk & 3) * 8; }
+
+// ------------------------------------------------------------------------------------------------
+// kernel 1: dK / dV.  One CTA owns a 128-row K/V tile of one kv head and walks the 128-row query tiles of every query head in its
+// group.  TMEM: S^T, dP^T, dV, dK of 128 columns each.  P^T and dS^T are fed to the MMA from TMEM.
 // ------------------------------------------------------------------------------------------------
 template <int D>
-struct BwdSmem {
-  static constexpr int BIG = 128 * D * 2;     // resident 128-row tile
-  static constexpr int SMALL = 64 * D * 2;    // streamed 64-row tile
-  static constexpr int STAGES = 4;
-  static constexpr int A_OFF = 0;             // resident tile 0 (K or Q)
-  static constexpr int B_OFF = BIG;           // resident tile 1 (V or dO)
-  static constexpr int S0_OFF = 2 * BIG;      // streamed tile 0 ring (Q or K)
-  static constexpr int S1_OFF = S0_OFF + STAGES * SMALL;   // streamed tile 1 ring (dO or V)
-  static constexpr int VEC_OFF = S1_OFF + STAGES * SMALL;  // per stage: 64 x (lse * log2e, delta) float pairs
-  static constexpr int BAR_OFF = VEC_OFF + STAGES * 512;
-  static constexpr int TOTAL = BAR_OFF + 256 + 1024;
+struct DkvSmem {
+  static constexpr int TILE = 128 * D * 2;
+  static constexpr int Q_STAGES = 3, DO_STAGES = 2;                   // Q(i + 1) is wanted while Q(i) waits for dK's product
+  static constexpr int K_OFF = 0, V_OFF = TILE;                       // resident
+  static constexpr int Q_OFF = 2 * TILE, DO_OFF = Q_OFF + Q_STAGES * TILE;   // streamed
+  static constexpr int VEC_OFF = DO_OFF + DO_STAGES * TILE;           // two of: 128 x lse * log2e, 128 x delta
+  static constexpr int BAR_OFF = VEC_OFF + 2 * 1024;
+  static constexpr int TOTAL = BAR_OFF + 256;                         // (no room for slack: the block itself is aligned)
 };
-
-constexpr int BWD_THREADS = 320;   // warp 0 TMA, warp 1 MMA, warps 2..5 and 6..9: two compute warpgroups (32 columns each)
-
-__device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
 
 template <int D, bool EXT>   // EXT: sliding window / logit soft-cap code paths compiled in
 __global__ void __launch_bounds__(BWD_THREADS, 1)
-flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ64, const __grid_constant__ CUtensorMap tmK128,
-                      const __grid_constant__ CUtensorMap tmV128, const __grid_constant__ CUtensorMap tmdO64,
-                      AttnParams p) {
-  using SM = BwdSmem<D>;
+flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+                      const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO, AttnParams p) {
+  using SM = DkvSmem<D>;
   constexpr int DCH = D / 64;
-  constexpr int STAGES = SM::STAGES;
   constexpr uint32_t TMEM_COLS = 512;
-  constexpr uint32_t DV_COL = 256, DK_COL = 384;
+  constexpr uint32_t DP_COL = 128, DV_COL = 256, DK_COL = 384;
 
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  float* vec = reinterpret_cast<float*>(smem + SM::VEC_OFF);   // [STAGES][64] (lse * log2e, delta) pairs
+  extern __shared__ __align__(1024) uint8_t smem_aligned[];
+  uint8_t* smem = smem_aligned;
+  if (smem_u32(smem) & 1023u) {            // the swizzled tiles need it
+    if (threadIdx.x == 0) ts_report_error(ERR_BAD_ARGUMENT, 730);
+    return;
+  }
+  float* vec = reinterpret_cast<float*>(smem + SM::VEC_OFF);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SM::BAR_OFF);
-  uint64_t* kv_full = bars;            // [1]
-  uint64_t* s_full = bars + 1;         // [2]
-  uint64_t* p_full = bars + 3;         // [2]
-  uint64_t* acc_full = bars + 5;       // [1]
-  uint64_t* qd_full = bars + 6;        // [STAGES]
-  uint64_t* qd_empty = bars + 6 + SM::STAGES;   // [STAGES]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 6 + 2 * SM::STAGES);
+  uint64_t* kv_full = bars;
+  uint64_t* s_full = bars + 1;
+  uint64_t* p_full = bars + 2;
+  uint64_t* dp_full = bars + 3;
+  uint64_t* ds_full = bars + 4;
+  uint64_t* acc_full = bars + 5;
+  uint64_t* q_full = bars + 6;      // [3]
+  uint64_t* q_empty = bars + 9;     // [3]
+  uint64_t* do_full = bars + 12;    // [2]
+  uint64_t* do_empty = bars + 14;   // [2]
+  uint64_t* vec_full = bars + 16;   // [2]
+  uint64_t* vec_empty = bars + 18;  // [2]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // grid: x = kv head + kv heads * batch (fastest), y = kv tile; low tiles see the most queries and go first
@@ -432,20 +465,19 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ64, const __grid_co
   const int k_start = q_start, Lk = Lq;
   if (j * 128 >= Lk) return;
   const int off = Lk - Lq;
-  const int n_u = (Lq + 63) / 64;
-  const int u_start = p.causal ? max(0, (j * 128 - off) / 64) : 0;
+  const int n_u = (Lq + 127) / 128;
+  const int u_start = p.causal ? max(0, (j * 128 - off) / 128) : 0;
   // sliding window: the last query row that sees any key of this tile is (j*128 + 127) - off + window - 1
-  const int u_end = (EXT && p.window > 0) ? min(n_u, (j * 128 + 127 - off + p.window - 1) / 64 + 1) : n_u;
+  const int u_end = (EXT && p.window > 0) ? min(n_u, (j * 128 + 127 - off + p.window - 1) / 128 + 1) : n_u;
   const int per_head = u_end - u_start;
   const int total = per_head * p.group;
 
   if (threadIdx.x == 0) {
-    tma_prefetch_desc(&tmQ64);
-    tma_prefetch_desc(&tmK128);
-    tma_prefetch_desc(&tmV128);
-    tma_prefetch_desc(&tmdO64);
-    for (int i = 0; i < 6 + 2 * SM::STAGES; ++i)
-      mbar_init(&bars[i], (i == 3 || i == 4) ? 8 : ((i >= 6 && i < 6 + SM::STAGES) ? 2 : 1));
+    tma_prefetch_desc(&tmQ);
+    tma_prefetch_desc(&tmK);
+    tma_prefetch_desc(&tmV);
+    tma_prefetch_desc(&tmdO);
+    for (int i = 0; i < 20; ++i) mbar_init(&bars[i], (i == 2 || i == 4 || i >= 18) ? 8 : 1);
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -459,204 +491,230 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ64, const __grid_co
   bool alive = true;
 
   if (warp == 0) {
-    // the whole warp runs the producer loop: lane 0 issues the tiled loads, every lane brings two columns'
-    // (lse * log2e, delta) pairs of the sub-tile into the stage's vector buffer (fetched one stage ahead)
+    // the whole warp runs the producer loop: lane 0 issues the tiled loads, every lane brings four columns' lse * log2e and
+    // delta into the stage's vector buffer (fetched one stage ahead)
     if (lane == 0) {
-      mbar_expect_tx(kv_full, 2 * SM::BIG);
+      mbar_expect_tx(kv_full, 2 * SM::TILE);
 #pragma unroll
       for (int c = 0; c < DCH; ++c) {
-        tma_load_2d(smem + SM::A_OFF + c * 16384, &tmK128, kv_full, p.k_col0 + hk * D + c * 64, k_start + j * 128);
-        tma_load_2d(smem + SM::B_OFF + c * 16384, &tmV128, kv_full, p.v_col0 + hk * D + c * 64, k_start + j * 128);
+        tma_load_2d(smem + SM::K_OFF + c * 16384, &tmK, kv_full, p.k_col0 + hk * D + c * 64, k_start + j * 128);
+        tma_load_2d(smem + SM::V_OFF + c * 16384, &tmV, kv_full, p.v_col0 + hk * D + c * 64, k_start + j * 128);
       }
     }
-    auto fetch_vec = [&](int it, int col) -> float2 {
+    float nl[4], nd[4];
+    auto fetch_vec = [&](int it) {
       const int g = it / per_head, u = u_start + it % per_head;
-      const int h = hk * p.group + g;
-      const int qrow = u * 64 + col;
-      if (it >= total || qrow >= Lq) return make_float2(0.f, 0.f);
-      const size_t idx = static_cast<size_t>(h) * p.total_rows + q_start + qrow;
-      return make_float2(p.lse[idx] * 1.4426950408889634f, p.delta[idx]);
-    };
-    float2 n0 = fetch_vec(0, lane), n1 = fetch_vec(0, lane + 32);
-    for (int it = 0; it < total && alive; ++it) {
-      const int s = it % STAGES;
-      const uint32_t ph = (it / STAGES) & 1u;
-      const int g = it / per_head, u = u_start + it % per_head;
-      const int h = hk * p.group + g;
-      if (!mbar_wait(&qd_empty[s], ph ^ 1u, alive, 700)) break;
-      if (lane == 0) {
-        mbar_expect_tx(&qd_full[s], 2 * SM::SMALL);
+      const size_t row0 = static_cast<size_t>(hk * p.group + g) * p.total_rows + q_start;
 #pragma unroll
-        for (int c = 0; c < DCH; ++c) {
-          tma_load_2d(smem + SM::S0_OFF + s * SM::SMALL + c * 8192, &tmQ64, &qd_full[s], p.q_col0 + h * D + c * 64,
-                      q_start + u * 64);
-          tma_load_2d(smem + SM::S1_OFF + s * SM::SMALL + c * 8192, &tmdO64, &qd_full[s], h * D + c * 64,
-                      q_start + u * 64);
-        }
+      for (int c = 0; c < 4; ++c) {
+        const int qrow = u * 128 + lane + c * 32;
+        const bool in = it < total && qrow < Lq;
+        nl[c] = in ? p.lse[row0 + qrow] * 1.4426950408889634f : 0.f;
+        nd[c] = in ? p.delta[row0 + qrow] : 0.f;
       }
-      float2* vb2 = reinterpret_cast<float2*>(vec + s * 128);
-      vb2[lane] = n0;
-      vb2[lane + 32] = n1;
-      n0 = fetch_vec(it + 1, lane);
-      n1 = fetch_vec(it + 1, lane + 32);
+    };
+    fetch_vec(0);
+    for (int it = 0; it < total && alive; ++it) {
+      const int s = it & 1, qs = it % SM::Q_STAGES;
+      const uint32_t ph = ((it >> 1) & 1u) ^ 1u;
+      const int u = u_start + it % per_head, h = hk * p.group + it / per_head;
+      if (!mbar_wait(&q_empty[qs], ((it / SM::Q_STAGES) & 1u) ^ 1u, alive, 700)) break;
+      if (lane == 0) {
+        mbar_expect_tx(&q_full[qs], SM::TILE);
+#pragma unroll
+        for (int c = 0; c < DCH; ++c)
+          tma_load_2d(smem + SM::Q_OFF + qs * SM::TILE + c * 16384, &tmQ, &q_full[qs], p.q_col0 + h * D + c * 64, q_start + u * 128);
+      }
+      if (!mbar_wait(&vec_empty[s], ph, alive, 702)) break;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        vec[s * 256 + lane + c * 32] = nl[c];
+        vec[s * 256 + 128 + lane + c * 32] = nd[c];
+      }
       __syncwarp();
-      if (lane == 0) mbar_arrive(&qd_full[s]);   // second arrival of the phase: the vectors are in place
+      if (lane == 0) mbar_arrive(&vec_full[s]);
+      fetch_vec(it + 1);
+      if (!mbar_wait(&do_empty[s], ph, alive, 701)) break;
+      if (lane == 0) {
+        mbar_expect_tx(&do_full[s], SM::TILE);
+#pragma unroll
+        for (int c = 0; c < DCH; ++c)
+          tma_load_2d(smem + SM::DO_OFF + s * SM::TILE + c * 16384, &tmdO, &do_full[s], h * D + c * 64, q_start + u * 128);
+      }
+      __syncwarp();
     }
   } else if (warp == 1) {
     if (elect_one_sync()) {
-      const uint32_t idesc_s = make_idesc(128, 64, 1, 1, 0, 0);
+      const uint32_t idesc_s = make_idesc(128, 128, 1, 1, 0, 0);
       const uint32_t idesc_acc = make_idesc(128, D, 1, 1, 0, 1);
-      const uint32_t ka = smem_u32(smem + SM::A_OFF), va = smem_u32(smem + SM::B_OFF);
-      auto issue12 = [&](int it) {
-        const int s = it % STAGES;
-        if (!mbar_wait(&qd_full[s], (it / STAGES) & 1u, alive, 710)) return;
-        tc_fence_after_sync();
-        const uint32_t qa = smem_u32(smem + SM::S0_OFF + s * SM::SMALL);
-        const uint32_t da = smem_u32(smem + SM::S1_OFF + s * SM::SMALL);
-        const uint32_t st = tmem_base + (it & 1) * 128;
+      // a (resident) times b (streamed), both K-major
+      auto issue_ss = [&](uint32_t d_col, uint32_t a, uint32_t bb) {
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
-          const uint32_t oa = (k >> 2) * 16384 + (k & 3) * 32, ob = (k >> 2) * 8192 + (k & 3) * 32;
-          umma_f16_ss(st, make_smem_desc_sw128(ka + oa, 16, 1024), make_smem_desc_sw128(qa + ob, 16, 1024), idesc_s,
+          const uint32_t o = (k >> 2) * 16384 + (k & 3) * 32;
+          umma_f16_ss(tmem_base + d_col, make_smem_desc_sw128(a + o, 16, 1024), make_smem_desc_sw128(bb + o, 16, 1024), idesc_s,
                       k != 0);
         }
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t oa = (k >> 2) * 16384 + (k & 3) * 32, ob = (k >> 2) * 8192 + (k & 3) * 32;
-          umma_f16_ss(st + 64, make_smem_desc_sw128(va + oa, 16, 1024), make_smem_desc_sw128(da + ob, 16, 1024),
-                      idesc_s, k != 0);
-        }
-        umma_commit(&s_full[it & 1]);
       };
-      if (mbar_wait(kv_full, 0, alive, 711)) {
-        issue12(0);
-        if (total > 1 && alive) issue12(1);
-        for (int it = 0; it < total && alive; ++it) {
-          const int bsel = it & 1, s = it % STAGES;
-          if (!mbar_wait(&p_full[bsel], (it >> 1) & 1u, alive, 712)) break;
+      auto issue_ts = [&](uint32_t d_col, uint32_t a_col, uint32_t bb, bool add) {
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk)
+          umma_f16_ts(tmem_base + d_col, tmem_base + a_col + half_col(kk), make_smem_desc_sw128(bb + kk * 2048, 16384, 1024),
+                      idesc_acc, add || kk != 0);
+      };
+      const uint32_t ka = smem_u32(smem + SM::K_OFF), va = smem_u32(smem + SM::V_OFF);
+      const uint32_t qa = smem_u32(smem + SM::Q_OFF), da = smem_u32(smem + SM::DO_OFF);
+      if (mbar_wait(kv_full, 0, alive, 710) && mbar_wait(&q_full[0], 0, alive, 711)) {
+        tc_fence_after_sync();
+        issue_ss(0, ka, qa);
+        umma_commit(s_full);
+        if (mbar_wait(&do_full[0], 0, alive, 712)) {
           tc_fence_after_sync();
-          const uint32_t qa = smem_u32(smem + SM::S0_OFF + s * SM::SMALL);
-          const uint32_t da = smem_u32(smem + SM::S1_OFF + s * SM::SMALL);
-          const uint32_t st = tmem_base + bsel * 128;
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            umma_f16_ts(tmem_base + DV_COL, st + (kk >> 1) * 32 + (kk & 1) * 8,
-                        make_smem_desc_sw128(da + kk * 2048, 8192, 1024), idesc_acc, (it | kk) != 0);
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            umma_f16_ts(tmem_base + DK_COL, st + 64 + (kk >> 1) * 32 + (kk & 1) * 8,
-                        make_smem_desc_sw128(qa + kk * 2048, 8192, 1024), idesc_acc, (it | kk) != 0);
-          umma_commit(&qd_empty[s]);
-          if (it + 2 < total) issue12(it + 2);
+          issue_ss(DP_COL, va, da);
+          umma_commit(dp_full);
         }
-        if (alive) umma_commit(acc_full);
       }
+      for (int it = 0; it < total && alive; ++it) {
+        const int s = it & 1, sn = s ^ 1, qs = it % SM::Q_STAGES, qn = (it + 1) % SM::Q_STAGES;
+        if (!mbar_wait(p_full, it & 1u, alive, 713)) break;
+        tc_fence_after_sync();
+        issue_ts(DV_COL, 0, da + s * SM::TILE, it != 0);
+        umma_commit(&do_empty[s]);
+        if (it + 1 < total) {
+          if (!mbar_wait(&q_full[qn], ((it + 1) / SM::Q_STAGES) & 1u, alive, 714)) break;
+          tc_fence_after_sync();
+          issue_ss(0, ka, qa + qn * SM::TILE);       // over P^T, which dV has read by then (products run in order)
+          umma_commit(s_full);
+        }
+        if (!mbar_wait(ds_full, it & 1u, alive, 715)) break;
+        tc_fence_after_sync();
+        issue_ts(DK_COL, DP_COL, qa + qs * SM::TILE, it != 0);
+        umma_commit(&q_empty[qs]);
+        if (it + 1 < total) {
+          if (!mbar_wait(&do_full[sn], ((it + 1) >> 1) & 1u, alive, 716)) break;
+          tc_fence_after_sync();
+          issue_ss(DP_COL, va, da + sn * SM::TILE);
+          umma_commit(dp_full);
+        }
+      }
+      if (alive) umma_commit(acc_full);
     }
   } else {
     const int q4 = warp & 3;
-    const int wg = (warp - 2) >> 2;          // compute warpgroup: owns query columns [wg*32, wg*32+32) of the sub-tile
+    const int wg = (warp - 2) >> 2;          // compute warpgroup: owns query columns [wg*64, wg*64+64) of the tile
     const int r = q4 * 32 + lane;            // kv row inside the tile
     const int kv_row = j * 128 + r;
     const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(q4 * 32) << 16);
+    const uint32_t t_s = t_lane + wg * 64, t_dp = t_lane + DP_COL + wg * 64;
     for (int it = 0; it < total && alive; ++it) {
       const int u = u_start + it % per_head;
-      // written by the producer warp before its arrival on qd_full, which the MMA thread observed before s_full
-      const float* vb = vec + (it % STAGES) * 128;
-      if (!mbar_wait(&s_full[it & 1], (it >> 1) & 1u, alive, 720)) break;
+      const float* lse2 = vec + (it & 1) * 256 + wg * 64;
+      const float* delta = lse2 + 128;
+      const int q0 = u * 128 + wg * 64;
+      const bool need_mask = (p.causal && (j * 128 + 127 > q0 + off)) || (q0 + 64 > Lq) || (j * 128 + 128 > Lk) ||
+                             (EXT && p.window > 0 && j * 128 <= q0 + 63 + off - p.window);
+      // visible columns of this row: [lo, hi)
+      int lo = 0, hi = 64;
+      if (need_mask) {
+        lo = p.causal ? max(0, kv_row - off - q0) : 0;
+        hi = kv_row < Lk ? min(64, Lq - q0) : 0;
+        if (EXT && p.window > 0) hi = min(hi, kv_row - off + p.window - q0);
+      }
+      if (!mbar_wait(&vec_full[it & 1], (it >> 1) & 1u, alive, 723)) break;
+      if (!mbar_wait(s_full, it & 1u, alive, 720)) break;
       tc_fence_after_sync();
-      const uint32_t t_s = t_lane + (it & 1) * 128;
-      const bool need_mask = (p.causal && (j * 128 + 127 > u * 64 + off)) || (u * 64 + 64 > Lq) ||
-                             (j * 128 + 128 > Lk) || (EXT && p.window > 0 && j * 128 <= u * 64 + 63 + off - p.window);
-      {
-        const int cc = wg;
-        uint32_t sv[32], dv[32], pp[16], ds[16];
-        tmem_ld_32x32b_x32(t_s + cc * 32, sv);
-        tmem_ld_32x32b_x32(t_s + 64 + cc * 32, dv);
-        tc_wait_ld();
-        // the masked and the unmasked tile bodies are separate straight-line code: a per-element branch would
-        // serialise the 32 independent exp chains
-        auto body = [&](auto masked, auto capped) {
+      uint32_t pv[64];                       // S, then P (times the soft cap's derivative), fp32
 #pragma unroll
-          for (int e = 0; e < 32; e += 2) {
-            const float4 ld4 = *reinterpret_cast<const float4*>(vb + 2 * (cc * 32 + e));   // warp-wide broadcast
-            float p0, p1, g0 = 1.f, g1 = 1.f;   // g = d(capped logit) / d(scaled logit)
-            if constexpr (decltype(capped)::value) {
-              const float t0 = fast_tanh(__uint_as_float(sv[e]) * p.cap_inv);
-              const float t1 = fast_tanh(__uint_as_float(sv[e + 1]) * p.cap_inv);
-              p0 = fast_ex2(fmaf(t0, p.cap_log2, -ld4.x));
-              p1 = fast_ex2(fmaf(t1, p.cap_log2, -ld4.z));
-              g0 = 1.f - t0 * t0;
-              g1 = 1.f - t1 * t1;
-            } else {
-              p0 = fast_ex2(fmaf(__uint_as_float(sv[e]), p.scale_log2, -ld4.x));
-              p1 = fast_ex2(fmaf(__uint_as_float(sv[e + 1]), p.scale_log2, -ld4.z));
+      for (int c = 0; c < 2; ++c) tmem_ld_32x32b_x32(t_s + c * 32, pv + c * 32);
+      tc_wait_ld();
+      const uint64_t sc2 = pack_f32x2(p.scale_log2, p.scale_log2);
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t pk[16];
+#pragma unroll
+        for (int e = 0; e < 32; e += 4) {
+          const int x = c * 32 + e;
+          const float4 l4 = *reinterpret_cast<const float4*>(lse2 + x);   // warp-wide broadcast
+          float v[4];
+          if (EXT && p.cap_log2 > 0.f) {
+            const float lv[4] = {l4.x, l4.y, l4.z, l4.w};
+#pragma unroll
+            for (int y = 0; y < 4; ++y) {
+              const float t = fast_tanh(__uint_as_float(pv[x + y]) * p.cap_inv);
+              v[y] = fast_ex2(fmaf(t, p.cap_log2, -lv[y]));
+              if (x + y < lo || x + y >= hi) v[y] = 0.f;
+              pv[x + y] = __float_as_uint(v[y] * (1.f - t * t));   // d(capped logit) / d(scaled logit)
             }
-            if constexpr (decltype(masked)::value) {
-              const int qrow = u * 64 + cc * 32 + e;
-              const bool rok = kv_row < Lk;
-              p0 = (rok && qrow < Lq && (!p.causal || kv_row <= qrow + off)) ? p0 : 0.f;
-              p1 = (rok && qrow + 1 < Lq && (!p.causal || kv_row <= qrow + 1 + off)) ? p1 : 0.f;
-              if constexpr (EXT) {   // sliding window: visible iff kv_row > qrow + off - window
-                if (p.window > 0) {
-                  p0 = (kv_row > qrow + off - p.window) ? p0 : 0.f;
-                  p1 = (kv_row > qrow + 1 + off - p.window) ? p1 : 0.f;
-                }
-              }
-            }
-            pp[e >> 1] = pack_bf16x2(p0, p1);
-            if constexpr (decltype(capped)::value)
-              ds[e >> 1] = pack_bf16x2(p0 * g0 * (__uint_as_float(dv[e]) - ld4.y),
-                                       p1 * g1 * (__uint_as_float(dv[e + 1]) - ld4.w));
-            else
-              ds[e >> 1] = pack_bf16x2(p0 * (__uint_as_float(dv[e]) - ld4.y), p1 * (__uint_as_float(dv[e + 1]) - ld4.w));
+          } else {
+            const float2 a = unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(pv[x]), __uint_as_float(pv[x + 1])), sc2,
+                                                    pack_f32x2(-l4.x, -l4.y)));
+            const float2 bq = unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(pv[x + 2]), __uint_as_float(pv[x + 3])), sc2,
+                                                     pack_f32x2(-l4.z, -l4.w)));
+            v[0] = fast_ex2(a.x);
+            v[1] = fast_ex2(a.y);
+            v[2] = fast_ex2(bq.x);
+            v[3] = fast_ex2(bq.y);
+#pragma unroll
+            for (int y = 0; y < 4; ++y) pv[x + y] = __float_as_uint(v[y]);
           }
-        };
-        if (EXT && p.cap_log2 > 0.f) body(std::true_type{}, std::true_type{});   // soft-cap: one (masked) variant only
-        else if (need_mask) body(std::true_type{}, std::false_type{});
-        else body(std::false_type{}, std::false_type{});
-        // each warpgroup overwrites only columns of its own (already consumed) chunk
-        tmem_st_32x32b_x16(t_s + cc * 32, pp);
-        tmem_st_32x32b_x16(t_s + 64 + cc * 32, ds);
+          pk[e >> 1] = pack_bf16x2(v[0], v[1]);
+          pk[(e >> 1) + 1] = pack_bf16x2(v[2], v[3]);
+        }
+        if (need_mask && !(EXT && p.cap_log2 > 0.f)) {
+#pragma unroll
+          for (int e = 0; e < 32; ++e)
+            if (c * 32 + e < lo || c * 32 + e >= hi) pv[c * 32 + e] = 0u;
+#pragma unroll
+          for (int e = 0; e < 32; e += 2)
+            pk[e >> 1] = pack_bf16x2(__uint_as_float(pv[c * 32 + e]), __uint_as_float(pv[c * 32 + e + 1]));
+        }
+        tmem_st_32x32b_x16(t_s + c * 16, pk);
       }
       tc_wait_st();
       tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full[it & 1]);
+      if (lane == 0) mbar_arrive(p_full);
+
+      if (!mbar_wait(dp_full, it & 1u, alive, 721)) break;
+      tc_fence_after_sync();
+      uint32_t ds[32];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t dv[32];
+        tmem_ld_32x32b_x32(t_dp + c * 32, dv);
+        tc_wait_ld();
+#pragma unroll
+        for (int e = 0; e < 32; e += 4) {
+          const int x = c * 32 + e;
+          const float4 d4 = *reinterpret_cast<const float4*>(delta + x);
+          const float2 a = unpack_f32x2(mul_f32x2(pack_f32x2(__uint_as_float(pv[x]), __uint_as_float(pv[x + 1])),
+                                                  add_f32x2(pack_f32x2(__uint_as_float(dv[e]), __uint_as_float(dv[e + 1])),
+                                                            pack_f32x2(-d4.x, -d4.y))));
+          const float2 bq = unpack_f32x2(mul_f32x2(pack_f32x2(__uint_as_float(pv[x + 2]), __uint_as_float(pv[x + 3])),
+                                                   add_f32x2(pack_f32x2(__uint_as_float(dv[e + 2]), __uint_as_float(dv[e + 3])),
+                                                             pack_f32x2(-d4.z, -d4.w))));
+          ds[x >> 1] = pack_bf16x2(a.x, a.y);
+          ds[(x >> 1) + 1] = pack_bf16x2(bq.x, bq.y);
+        }
+      }
+      tmem_st_32x32b_x32(t_dp, ds);
+      tc_wait_st();
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&vec_empty[it & 1]);
+        mbar_arrive(ds_full);
+      }
     }
-    if (alive && mbar_wait(acc_full, 0, alive, 721)) {
+    if (alive && mbar_wait(acc_full, 0, alive, 722)) {
       tc_fence_after_sync();
       const bool valid = kv_row < Lk;
       __nv_bfloat16* dvp = p.dv + static_cast<size_t>(k_start + kv_row) * p.dqkv_stride + p.v_col0 + hk * D;
       __nv_bfloat16* dkp = p.dk + static_cast<size_t>(k_start + kv_row) * p.dqkv_stride + p.k_col0 + hk * D;
 #pragma unroll 1
       for (int c = wg; c < D / 32; c += 2) {
-        uint32_t v[32];
-        tmem_ld_32x32b_x32(t_lane + DV_COL + c * 32, v);
-        tc_wait_ld();
-        if (valid) {
-#pragma unroll
-          for (int x = 0; x < 4; ++x) {
-            uint4 o4;
-            o4.x = pack_bf16x2(__uint_as_float(v[8 * x]), __uint_as_float(v[8 * x + 1]));
-            o4.y = pack_bf16x2(__uint_as_float(v[8 * x + 2]), __uint_as_float(v[8 * x + 3]));
-            o4.z = pack_bf16x2(__uint_as_float(v[8 * x + 4]), __uint_as_float(v[8 * x + 5]));
-            o4.w = pack_bf16x2(__uint_as_float(v[8 * x + 6]), __uint_as_float(v[8 * x + 7]));
-            *reinterpret_cast<uint4*>(dvp + c * 32 + x * 8) = o4;
-          }
-        }
-        tmem_ld_32x32b_x32(t_lane + DK_COL + c * 32, v);
-        tc_wait_ld();
-        if (valid) {
-#pragma unroll
-          for (int x = 0; x < 4; ++x) {
-            uint4 o4;
-            o4.x = pack_bf16x2(__uint_as_float(v[8 * x]) * p.scale, __uint_as_float(v[8 * x + 1]) * p.scale);
-            o4.y = pack_bf16x2(__uint_as_float(v[8 * x + 2]) * p.scale, __uint_as_float(v[8 * x + 3]) * p.scale);
-            o4.z = pack_bf16x2(__uint_as_float(v[8 * x + 4]) * p.scale, __uint_as_float(v[8 * x + 5]) * p.scale);
-            o4.w = pack_bf16x2(__uint_as_float(v[8 * x + 6]) * p.scale, __uint_as_float(v[8 * x + 7]) * p.scale);
-            *reinterpret_cast<uint4*>(dkp + c * 32 + x * 8) = o4;
-          }
-        }
+        store_rows_32(t_lane + DV_COL + c * 32, 1.f, dvp + c * 32, valid);
+        store_rows_32(t_lane + DK_COL + c * 32, p.scale, dkp + c * 32, valid);
       }
     }
   }
@@ -669,30 +727,41 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ64, const __grid_co
 }
 
 // ------------------------------------------------------------------------------------------------
-// backward, kernel 2: dQ.  One CTA owns a 128-row query tile of one head (Q and dO resident) and walks the
-// 64-row K/V sub-tiles it can see.  TMEM: two (S | dP) buffers of 64+64 columns and the dQ accumulator.
+// kernel 2: dQ.  One CTA owns a 128-row query tile of one head (Q and dO resident) and walks the 128-row K/V tiles it can see.
+// TMEM: two S buffers, dP, dQ of 128 columns each.  Three K stages: K(i + 2) is wanted for S while K(i) is in dQ's product.
 // ------------------------------------------------------------------------------------------------
+template <int D>
+struct DqSmem {
+  static constexpr int TILE = 128 * D * 2;
+  static constexpr int K_STAGES = 3, V_STAGES = 2;
+  static constexpr int Q_OFF = 0, DO_OFF = TILE;
+  static constexpr int K_OFF = 2 * TILE, V_OFF = K_OFF + K_STAGES * TILE;
+  static constexpr int BAR_OFF = V_OFF + V_STAGES * TILE;
+  static constexpr int TOTAL = BAR_OFF + 256 + 1024;
+};
+
 template <int D, bool EXT>   // EXT: sliding window / logit soft-cap code paths compiled in
 __global__ void __launch_bounds__(BWD_THREADS, 1)
-flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ128, const __grid_constant__ CUtensorMap tmK64,
-                    const __grid_constant__ CUtensorMap tmV64, const __grid_constant__ CUtensorMap tmdO128,
-                    AttnParams p) {
-  using SM = BwdSmem<D>;
+flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO, AttnParams p) {
+  using SM = DqSmem<D>;
   constexpr int DCH = D / 64;
-  constexpr int STAGES = SM::STAGES;
   constexpr uint32_t TMEM_COLS = 512;
-  constexpr uint32_t DQ_COL = 256;
+  constexpr uint32_t DP_COL = 256, DQ_COL = 384;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SM::BAR_OFF);
-  uint64_t* q_full = bars;             // [1]
-  uint64_t* s_full = bars + 1;         // [2]
-  uint64_t* p_full = bars + 3;         // [2]
-  uint64_t* acc_full = bars + 5;       // [1]
-  uint64_t* kv_full = bars + 6;        // [STAGES]
-  uint64_t* kv_empty = bars + 6 + SM::STAGES;   // [STAGES]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 6 + 2 * SM::STAGES);
+  uint64_t* qd_full = bars;         // [1]
+  uint64_t* s_full = bars + 1;      // [2]
+  uint64_t* dp_full = bars + 3;     // [1]
+  uint64_t* ds_full = bars + 4;     // [1]
+  uint64_t* acc_full = bars + 5;    // [1]
+  uint64_t* k_full = bars + 6;      // [3]
+  uint64_t* k_empty = bars + 9;     // [3]
+  uint64_t* v_full = bars + 12;     // [2]
+  uint64_t* v_empty = bars + 14;    // [2]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // grid: x = head + heads * batch (fastest), y = tile: the whole grid is dispatched longest-tile-first
@@ -706,16 +775,16 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ128, const __grid_con
   const int i = n_qt - 1 - blockIdx.y;
   const int off = Lk - Lq;
   const int kv_end = p.causal ? min(Lk, i * 128 + 128 + off) : Lk;
-  // sliding window: 64-key sub-tiles entirely left of the first row's window are skipped
-  const int sub0 = (EXT && p.window > 0) ? max(0, i * 128 + off - p.window + 1) / 64 : 0;
-  const int total = (kv_end + 63) / 64 - sub0;
+  // sliding window: key tiles entirely left of the first row's window are skipped
+  const int tile0 = (EXT && p.window > 0) ? max(0, i * 128 + off - p.window + 1) / 128 : 0;
+  const int total = (kv_end + 127) / 128 - tile0;
 
   if (threadIdx.x == 0) {
-    tma_prefetch_desc(&tmQ128);
-    tma_prefetch_desc(&tmK64);
-    tma_prefetch_desc(&tmV64);
-    tma_prefetch_desc(&tmdO128);
-    for (int x = 0; x < 6 + 2 * SM::STAGES; ++x) mbar_init(&bars[x], (x == 3 || x == 4) ? 8 : 1);
+    tma_prefetch_desc(&tmQ);
+    tma_prefetch_desc(&tmK);
+    tma_prefetch_desc(&tmV);
+    tma_prefetch_desc(&tmdO);
+    for (int x = 0; x < 16; ++x) mbar_init(&bars[x], x == 4 ? 8 : 1);
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -730,66 +799,81 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ128, const __grid_con
 
   if (warp == 0) {
     if (elect_one_sync()) {
-      mbar_expect_tx(q_full, 2 * SM::BIG);
+      mbar_expect_tx(qd_full, 2 * SM::TILE);
 #pragma unroll
       for (int c = 0; c < DCH; ++c) {
-        tma_load_2d(smem + SM::A_OFF + c * 16384, &tmQ128, q_full, p.q_col0 + h * D + c * 64, q_start + i * 128);
-        tma_load_2d(smem + SM::B_OFF + c * 16384, &tmdO128, q_full, h * D + c * 64, q_start + i * 128);
+        tma_load_2d(smem + SM::Q_OFF + c * 16384, &tmQ, qd_full, p.q_col0 + h * D + c * 64, q_start + i * 128);
+        tma_load_2d(smem + SM::DO_OFF + c * 16384, &tmdO, qd_full, h * D + c * 64, q_start + i * 128);
       }
-      for (int it = 0; it < total && alive; ++it) {
-        const int s = it % STAGES;
-        if (!mbar_wait(&kv_empty[s], ((it / STAGES) & 1u) ^ 1u, alive, 800)) break;
-        mbar_expect_tx(&kv_full[s], 2 * SM::SMALL);
+      // in the order the products want them: K(0) V(0) K(1), then V(i), K(i + 1)
+      auto load_k = [&](int it) {
+        const int s = it % SM::K_STAGES;
+        if (!mbar_wait(&k_empty[s], ((it / SM::K_STAGES) & 1u) ^ 1u, alive, 800)) return;
+        mbar_expect_tx(&k_full[s], SM::TILE);
 #pragma unroll
-        for (int c = 0; c < DCH; ++c) {
-          tma_load_2d(smem + SM::S0_OFF + s * SM::SMALL + c * 8192, &tmK64, &kv_full[s], p.k_col0 + hk * D + c * 64,
-                      k_start + (sub0 + it) * 64);
-          tma_load_2d(smem + SM::S1_OFF + s * SM::SMALL + c * 8192, &tmV64, &kv_full[s], p.v_col0 + hk * D + c * 64,
-                      k_start + (sub0 + it) * 64);
-        }
+        for (int c = 0; c < DCH; ++c)
+          tma_load_2d(smem + SM::K_OFF + s * SM::TILE + c * 16384, &tmK, &k_full[s], p.k_col0 + hk * D + c * 64,
+                      k_start + (tile0 + it) * 128);
+      };
+      auto load_v = [&](int it) {
+        const int s = it % SM::V_STAGES;
+        if (!mbar_wait(&v_empty[s], ((it / SM::V_STAGES) & 1u) ^ 1u, alive, 801)) return;
+        mbar_expect_tx(&v_full[s], SM::TILE);
+#pragma unroll
+        for (int c = 0; c < DCH; ++c)
+          tma_load_2d(smem + SM::V_OFF + s * SM::TILE + c * 16384, &tmV, &v_full[s], p.v_col0 + hk * D + c * 64,
+                      k_start + (tile0 + it) * 128);
+      };
+      if (total > 0) load_k(0);
+      for (int it = 0; it < total && alive; ++it) {
+        load_v(it);
+        if (it + 1 < total && alive) load_k(it + 1);
       }
     }
   } else if (warp == 1) {
     if (elect_one_sync()) {
-      const uint32_t idesc_s = make_idesc(128, 64, 1, 1, 0, 0);
+      const uint32_t idesc_s = make_idesc(128, 128, 1, 1, 0, 0);
       const uint32_t idesc_acc = make_idesc(128, D, 1, 1, 0, 1);
-      const uint32_t qa = smem_u32(smem + SM::A_OFF), da = smem_u32(smem + SM::B_OFF);
-      auto issue12 = [&](int it) {
-        const int s = it % STAGES;
-        if (!mbar_wait(&kv_full[s], (it / STAGES) & 1u, alive, 810)) return;
-        tc_fence_after_sync();
-        const uint32_t ka = smem_u32(smem + SM::S0_OFF + s * SM::SMALL);
-        const uint32_t va = smem_u32(smem + SM::S1_OFF + s * SM::SMALL);
-        const uint32_t st = tmem_base + (it & 1) * 128;
+      const uint32_t qa = smem_u32(smem + SM::Q_OFF), da = smem_u32(smem + SM::DO_OFF);
+      const uint32_t ka = smem_u32(smem + SM::K_OFF), va = smem_u32(smem + SM::V_OFF);
+      auto issue_ss = [&](uint32_t d_col, uint32_t a, uint32_t bb) {
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
-          const uint32_t oa = (k >> 2) * 16384 + (k & 3) * 32, ob = (k >> 2) * 8192 + (k & 3) * 32;
-          umma_f16_ss(st, make_smem_desc_sw128(qa + oa, 16, 1024), make_smem_desc_sw128(ka + ob, 16, 1024), idesc_s,
+          const uint32_t o = (k >> 2) * 16384 + (k & 3) * 32;
+          umma_f16_ss(tmem_base + d_col, make_smem_desc_sw128(a + o, 16, 1024), make_smem_desc_sw128(bb + o, 16, 1024), idesc_s,
                       k != 0);
         }
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t oa = (k >> 2) * 16384 + (k & 3) * 32, ob = (k >> 2) * 8192 + (k & 3) * 32;
-          umma_f16_ss(st + 64, make_smem_desc_sw128(da + oa, 16, 1024), make_smem_desc_sw128(va + ob, 16, 1024),
-                      idesc_s, k != 0);
-        }
+      };
+      auto issue_s = [&](int it) {
+        const int s = it % SM::K_STAGES;
+        if (!mbar_wait(&k_full[s], (it / SM::K_STAGES) & 1u, alive, 810)) return;
+        tc_fence_after_sync();
+        issue_ss((it & 1) * 128, qa, ka + s * SM::TILE);
         umma_commit(&s_full[it & 1]);
       };
-      if (mbar_wait(q_full, 0, alive, 811)) {
-        issue12(0);
-        if (total > 1 && alive) issue12(1);
+      auto issue_dp = [&](int it) {
+        const int s = it % SM::V_STAGES;
+        if (!mbar_wait(&v_full[s], (it / SM::V_STAGES) & 1u, alive, 811)) return;
+        tc_fence_after_sync();
+        issue_ss(DP_COL, da, va + s * SM::TILE);
+        umma_commit(dp_full);
+        umma_commit(&v_empty[s]);
+      };
+      if (total > 0 && mbar_wait(qd_full, 0, alive, 812)) {
+        issue_s(0);
+        if (alive) issue_dp(0);
+        if (total > 1 && alive) issue_s(1);
         for (int it = 0; it < total && alive; ++it) {
-          const int bsel = it & 1, s = it % STAGES;
-          if (!mbar_wait(&p_full[bsel], (it >> 1) & 1u, alive, 812)) break;
+          const int s = it % SM::K_STAGES;
+          if (!mbar_wait(ds_full, it & 1u, alive, 813)) break;
           tc_fence_after_sync();
-          const uint32_t ka = smem_u32(smem + SM::S0_OFF + s * SM::SMALL);
-          const uint32_t st = tmem_base + bsel * 128;
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            umma_f16_ts(tmem_base + DQ_COL, st + 64 + (kk >> 1) * 32 + (kk & 1) * 8,
-                        make_smem_desc_sw128(ka + kk * 2048, 8192, 1024), idesc_acc, (it | kk) != 0);
-          umma_commit(&kv_empty[s]);
-          if (it + 2 < total) issue12(it + 2);
+          for (int kk = 0; kk < 8; ++kk)
+            umma_f16_ts(tmem_base + DQ_COL, tmem_base + DP_COL + half_col(kk),
+                        make_smem_desc_sw128(ka + s * SM::TILE + kk * 2048, 16384, 1024), idesc_acc, (it | kk) != 0);
+          umma_commit(&k_empty[s]);
+          if (it + 1 < total) issue_dp(it + 1);                // over dS, which dQ has read by then
+          if (it + 2 < total && alive) issue_s(it + 2);        // S(it) was read before dS(it) was written
         }
         if (alive) umma_commit(acc_full);
       }
@@ -800,6 +884,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ128, const __grid_con
     const int r = q4 * 32 + lane;
     const int qrow = i * 128 + r;
     const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(q4 * 32) << 16);
+    const uint32_t t_dp = t_lane + DP_COL + wg * 64;
     float lse2 = 0.f, delta = 0.f;
     if (qrow < Lq) {
       const size_t idx = static_cast<size_t>(h) * p.total_rows + q_start + qrow;
@@ -807,82 +892,64 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ128, const __grid_con
       delta = p.delta[idx];
     }
     const int limit = (qrow < Lq) ? (p.causal ? min(Lk - 1, qrow + off) : Lk - 1) : -1;
-    const int lo = (EXT && p.window > 0) ? qrow + off - p.window + 1 : 0;
+    const int first = (EXT && p.window > 0) ? qrow + off - p.window + 1 : 0;
+    const uint64_t sc2 = pack_f32x2(p.scale_log2, p.scale_log2), ml2 = pack_f32x2(-lse2, -lse2), md2 = pack_f32x2(-delta, -delta);
     for (int it = 0; it < total && alive; ++it) {
+      const int col0 = (tile0 + it) * 128 + wg * 64;
+      const bool need_mask = (p.causal && col0 + 63 > i * 128 + off) || (col0 + 64 > Lk) || (i * 128 + 128 > Lq) ||
+                             (EXT && p.window > 0 && col0 <= i * 128 + 127 + off - p.window);
       if (!mbar_wait(&s_full[it & 1], (it >> 1) & 1u, alive, 820)) break;
       tc_fence_after_sync();
-      const uint32_t t_s = t_lane + (it & 1) * 128;
-      const int col0 = (sub0 + it) * 64;
-      const bool need_mask = (col0 + 63 > i * 128 + off && p.causal) || (col0 + 64 > Lk) || (i * 128 + 128 > Lq) ||
-                             (EXT && p.window > 0 && col0 <= i * 128 + 127 + off - p.window);
-      {
-        const int cc = wg;
-        uint32_t sv[32], dv[32], ds[16];
-        tmem_ld_32x32b_x32(t_s + cc * 32, sv);
-        tmem_ld_32x32b_x32(t_s + 64 + cc * 32, dv);
-        tc_wait_ld();
-        auto body = [&](auto masked, auto capped) {
+      uint32_t pv[64];
 #pragma unroll
-          for (int e = 0; e < 32; e += 2) {
-            float p0, p1, g0 = 1.f, g1 = 1.f;
-            if constexpr (decltype(capped)::value) {
-              const float t0 = fast_tanh(__uint_as_float(sv[e]) * p.cap_inv);
-              const float t1 = fast_tanh(__uint_as_float(sv[e + 1]) * p.cap_inv);
-              p0 = fast_ex2(fmaf(t0, p.cap_log2, -lse2));
-              p1 = fast_ex2(fmaf(t1, p.cap_log2, -lse2));
-              g0 = 1.f - t0 * t0;
-              g1 = 1.f - t1 * t1;
-            } else {
-              p0 = fast_ex2(fmaf(__uint_as_float(sv[e]), p.scale_log2, -lse2));
-              p1 = fast_ex2(fmaf(__uint_as_float(sv[e + 1]), p.scale_log2, -lse2));
-            }
-            if constexpr (decltype(masked)::value) {
-              const int col = col0 + cc * 32 + e;
-              p0 = (col <= limit) ? p0 : 0.f;
-              p1 = (col + 1 <= limit) ? p1 : 0.f;
-              if constexpr (EXT) {
-                p0 = (col >= lo) ? p0 : 0.f;
-                p1 = (col + 1 >= lo) ? p1 : 0.f;
-              }
-            }
-            if constexpr (decltype(capped)::value)
-              ds[e >> 1] = pack_bf16x2(p0 * g0 * (__uint_as_float(dv[e]) - delta),
-                                       p1 * g1 * (__uint_as_float(dv[e + 1]) - delta));
-            else
-              ds[e >> 1] = pack_bf16x2(p0 * (__uint_as_float(dv[e]) - delta), p1 * (__uint_as_float(dv[e + 1]) - delta));
-          }
-        };
-        if (EXT && p.cap_log2 > 0.f) body(std::true_type{}, std::true_type{});
-        else if (need_mask) body(std::true_type{}, std::false_type{});
-        else body(std::false_type{}, std::false_type{});
-        tmem_st_32x32b_x16(t_s + 64 + cc * 32, ds);
+      for (int c = 0; c < 2; ++c) tmem_ld_32x32b_x32(t_lane + (it & 1) * 128 + wg * 64 + c * 32, pv + c * 32);
+      tc_wait_ld();
+      if (EXT && p.cap_log2 > 0.f) {
+#pragma unroll
+        for (int e = 0; e < 64; ++e) {
+          const float t = fast_tanh(__uint_as_float(pv[e]) * p.cap_inv);
+          pv[e] = __float_as_uint(fast_ex2(fmaf(t, p.cap_log2, -lse2)) * (1.f - t * t));
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < 64; e += 2) {
+          const float2 a = unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(pv[e]), __uint_as_float(pv[e + 1])), sc2, ml2));
+          pv[e] = __float_as_uint(fast_ex2(a.x));
+          pv[e + 1] = __float_as_uint(fast_ex2(a.y));
+        }
       }
+      if (need_mask) {
+#pragma unroll
+        for (int e = 0; e < 64; ++e)
+          if (col0 + e > limit || (EXT && col0 + e < first)) pv[e] = 0u;
+      }
+      if (!mbar_wait(dp_full, it & 1u, alive, 821)) break;
+      tc_fence_after_sync();
+      uint32_t ds[32];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t dv[32];
+        tmem_ld_32x32b_x32(t_dp + c * 32, dv);
+        tc_wait_ld();
+#pragma unroll
+        for (int e = 0; e < 32; e += 2) {
+          const int x = c * 32 + e;
+          const float2 a = unpack_f32x2(mul_f32x2(pack_f32x2(__uint_as_float(pv[x]), __uint_as_float(pv[x + 1])),
+                                                  add_f32x2(pack_f32x2(__uint_as_float(dv[e]), __uint_as_float(dv[e + 1])), md2)));
+          ds[x >> 1] = pack_bf16x2(a.x, a.y);
+        }
+      }
+      tmem_st_32x32b_x32(t_dp, ds);
       tc_wait_st();
       tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full[it & 1]);
+      if (lane == 0) mbar_arrive(ds_full);
     }
-    if (alive && mbar_wait(acc_full, 0, alive, 821)) {
+    if (total > 0 && alive && mbar_wait(acc_full, 0, alive, 822)) {
       tc_fence_after_sync();
-      const bool valid = qrow < Lq;
       __nv_bfloat16* dqp = p.dq + static_cast<size_t>(q_start + qrow) * p.dqkv_stride + p.q_col0 + h * D;
 #pragma unroll 1
-      for (int c = wg; c < D / 32; c += 2) {
-        uint32_t v[32];
-        tmem_ld_32x32b_x32(t_lane + DQ_COL + c * 32, v);
-        tc_wait_ld();
-        if (valid) {
-#pragma unroll
-          for (int x = 0; x < 4; ++x) {
-            uint4 o4;
-            o4.x = pack_bf16x2(__uint_as_float(v[8 * x]) * p.scale, __uint_as_float(v[8 * x + 1]) * p.scale);
-            o4.y = pack_bf16x2(__uint_as_float(v[8 * x + 2]) * p.scale, __uint_as_float(v[8 * x + 3]) * p.scale);
-            o4.z = pack_bf16x2(__uint_as_float(v[8 * x + 4]) * p.scale, __uint_as_float(v[8 * x + 5]) * p.scale);
-            o4.w = pack_bf16x2(__uint_as_float(v[8 * x + 6]) * p.scale, __uint_as_float(v[8 * x + 7]) * p.scale);
-            *reinterpret_cast<uint4*>(dqp + c * 32 + x * 8) = o4;
-          }
-        }
-      }
+      for (int c = wg; c < D / 32; c += 2) store_rows_32(t_lane + DQ_COL + c * 32, p.scale, dqp + c * 32, qrow < Lq);
     }
   }
   tc_fence_before_sync();
@@ -898,17 +965,17 @@ static int launch_bwd(const CUtensorMap* m, const AttnParams& p, int max_len, cu
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(flash_bwd_dkdv_kernel<D, EXT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         BwdSmem<D>::TOTAL);
+                                         DkvSmem<D>::TOTAL);
     if (e != cudaSuccess) return (int)e;
-    e = cudaFuncSetAttribute(flash_bwd_dq_kernel<D, EXT>, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<D>::TOTAL);
+    e = cudaFuncSetAttribute(flash_bwd_dq_kernel<D, EXT>, cudaFuncAttributeMaxDynamicSharedMemorySize, DqSmem<D>::TOTAL);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  // m: [0]=q64 [1]=k128 [2]=v128 [3]=do64 [4]=q128 [5]=k64 [6]=v64 [7]=do128
+  // m: q, k, v, dO
   dim3 g1(p.Hkv * p.B, (max_len + 127) / 128, 1);
-  flash_bwd_dkdv_kernel<D, EXT><<<g1, BWD_THREADS, BwdSmem<D>::TOTAL, st>>>(m[0], m[1], m[2], m[3], p);
+  flash_bwd_dkdv_kernel<D, EXT><<<g1, BWD_THREADS, DkvSmem<D>::TOTAL, st>>>(m[0], m[1], m[2], m[3], p);
   dim3 g2(p.Hq * p.B, (max_len + 127) / 128, 1);
-  flash_bwd_dq_kernel<D, EXT><<<g2, BWD_THREADS, BwdSmem<D>::TOTAL, st>>>(m[4], m[5], m[6], m[7], p);
+  flash_bwd_dq_kernel<D, EXT><<<g2, BWD_THREADS, DqSmem<D>::TOTAL, st>>>(m[0], m[1], m[2], m[3], p);
   return (int)cudaGetLastError();
 }
 
@@ -1015,17 +1082,13 @@ extern "C" int ts_flash_bwd_ex(const void* q, const void* k, const void* v, cons
                                const int* cu_seqlens, int max_len, int causal, float scale, int window, float softcap,
                                void* stream) {
   if ((D != 64 && D != 128) || Hq % Hkv != 0 || total_rows <= 0) return -10;
-  CUtensorMap m[8];
+  CUtensorMap m[4];
   const void* bases[4] = {q, k, v, dout};
   const int strides[4] = {qkv_stride, qkv_stride, qkv_stride, o_stride};
-  const int small_first[4] = {1, 0, 0, 1};   // q, dO are streamed (64 rows) in the dK/dV kernel; k, v in the dQ kernel
   for (int t = 0; t < 4; ++t) {
     int rc = make_tmap_2d(&m[t], bases[t], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)total_rows,
-                          (uint64_t)strides[t], (uint64_t)strides[t], small_first[t] ? 64 : 128, 64);
+                          (uint64_t)strides[t], (uint64_t)strides[t], 128, 64);
     if (rc) return rc * 100 - 10 - t;
-    rc = make_tmap_2d(&m[4 + t], bases[t], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)total_rows,
-                      (uint64_t)strides[t], (uint64_t)strides[t], small_first[t] ? 128 : 64, 64);
-    if (rc) return rc * 100 - 20 - t;
   }
   AttnParams p{};
   p.q_col0 = q_col0; p.k_col0 = k_col0; p.v_col0 = v_col0;
