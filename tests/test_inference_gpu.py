@@ -213,3 +213,68 @@ def test_decode_attention_matches_fp64(Hq, Hkv, D, bs, lens, splits, chunk):
         ref = torch.einsum("hk,khd->hd", w, v).reshape(-1)
         err = (out[i].double() - ref).abs()
         assert (err <= 2.0 ** -8 * ref.abs() + 2.0 ** -15 * 5).all(), (i, float(err.max()))
+
+
+@pytest.mark.parametrize("D,Hq,Hkv", [(64, 4, 2), (128, 3, 1), (16, 20, 20)])
+@pytest.mark.parametrize("rows", [1, 37])
+def test_rotation_and_cache_write_in_one_launch(D, Hq, Hkv, rows):
+    """Against the separate rotation and a scatter; both round a * cos -+ b * sin to bf16 once (2^-8 of the operands)."""
+    import ctypes
+    from trainscale_b200.ops import _lib, rope
+    torch.manual_seed(0)
+    cos, sin = rope.rope_tables(512, D, device="cuda")
+    qkv = torch.randn(rows, (Hq + 2 * Hkv) * D, device="cuda").bfloat16()
+    pos = torch.randint(0, 512, (rows,), device="cuda", dtype=torch.int32)
+    slots = torch.randperm(64, device="cuda")[:rows].clone()
+    slots[-1] = -1 if rows > 1 else slots[-1]
+    want = rope.apply_rope_qkv(qkv.unsqueeze(0), Hq + Hkv, D, cos, sin, pos.unsqueeze(0), rows)[0]
+    kc, vc = (torch.full((64, Hkv * D), 7.0, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    got = qkv.clone()
+    rc = _lib.load("decode").ts_rope_cache(_lib.ptr(got), ctypes.c_longlong(got.stride(0)), _lib.ptr(cos), _lib.ptr(sin), _lib.ptr(pos),
+                                           _lib.ptr(slots), _lib.ptr(kc), _lib.ptr(vc), ctypes.c_longlong(rows), Hq, Hkv, D,
+                                           _lib.stream_ptr())
+    assert rc == 0
+    assert (got.float() - want.float()).abs().max() <= 2.0 ** -7 * 5
+    keep = slots >= 0
+    assert torch.equal(kc[slots[keep]], got[keep, Hq * D:(Hq + Hkv) * D]) and torch.equal(vc[slots[keep]], got[keep, (Hq + Hkv) * D:])
+    rest = torch.ones(64, dtype=torch.bool, device="cuda")
+    rest[slots[keep]] = False
+    assert (kc[rest] == 7.0).all() and (vc[rest] == 7.0).all()
+
+
+@pytest.mark.parametrize("H", [8, 264, 2048, 8192])
+@pytest.mark.parametrize("residual", [False, True])
+def test_norm_of_step_rows(H, residual):
+    """fp32 math on bf16 rows: one rounding of the result, beside a sum in another order (2^-8 covers both)."""
+    from trainscale_b200.ops import norm
+    torch.manual_seed(0)
+    for rows in (1, 5, norm.STEP_ROWS, norm.STEP_ROWS + 1):
+        x, r = (torch.randn(rows, H, device="cuda").bfloat16() for _ in range(2))
+        w = torch.randn(H, device="cuda").bfloat16()
+        y, h = norm.rmsnorm_step(x, w, 1e-5, r if residual else None, 1.0)
+        ref, href = norm.rmsnorm_reference(x.double().float(), w.float(), 1e-5, None, 1.0) if not residual else \
+            norm.rmsnorm_reference((x.float() + r.float()).bfloat16().float(), w.float(), 1e-5, None, 1.0)
+        assert torch.equal(h.float(), href)
+        assert ((y.float() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-6).all()
+
+
+def test_chained_steps_wait_for_their_rows():
+    """A chain of norm and products whose weights are fetched ahead gives the bits of the same kernels launched one by one."""
+    from trainscale_b200.ops import gemm, norm
+    torch.manual_seed(0)
+    H, I = 2048, 4096
+    w1, w2, nw = torch.randn(2 * I, H, device="cuda").bfloat16() * 0.02, torch.randn(H, I, device="cuda").bfloat16() * 0.02, torch.ones(H, device="cuda").bfloat16()
+    x = torch.randn(17, H, device="cuda").bfloat16()
+
+    def run(chained):
+        h, res = x, None
+        for _ in range(20):
+            n, res = norm.rmsnorm_step(h, nw, 1e-5, res)
+            if not chained:
+                torch.cuda.synchronize()
+            h = gemm.step_linear(gemm.step_glu(n, w1, "silu", chained=chained), w2, chained=chained)
+        return h
+
+    want = run(False)
+    for _ in range(5):
+        assert torch.equal(run(True), want)

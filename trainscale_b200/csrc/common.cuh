@@ -214,6 +214,15 @@ __device__ __forceinline__ float block_max(float v, float* scratch) {
 }
 
 // ---------------------------------------------------------------------------------------------
+// chained launches (host_common.h launch_chained): the kernel may start while its predecessor in the stream still runs.  Every
+// thread calls grid_wait before it touches anything an earlier kernel may have written or may still read, and grid_trigger only
+// after it, so that a kernel that starts early finds everything BEFORE its predecessor finished and visible: weights, which no
+// kernel of a step writes, can be fetched ahead of grid_wait.  Both do nothing in an ordinary launch.
+// ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// ---------------------------------------------------------------------------------------------
 // mbarrier
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {

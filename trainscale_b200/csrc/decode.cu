@@ -8,6 +8,51 @@
 
 namespace ts {
 
+// Rotary embedding (partners i and i + D / 2) of the q and k heads of projection rows, in place, and the cache write of the rotated
+// keys and the values: one launch and one pass instead of a copy of the rows, a rotation and a write.  One CTA per row: a thread
+// owns eight pairs of a head or eight values.
+constexpr int RC_THREADS = 256;
+__global__ void __launch_bounds__(RC_THREADS)
+rope_cache_kernel(__nv_bfloat16* __restrict__ qkv, long long row_stride, const float* __restrict__ cos_t,
+                  const float* __restrict__ sin_t, const int* __restrict__ pos, const long long* __restrict__ slot_mapping,
+                  __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache, int Hq, int Hkv, int D) {
+  grid_wait();
+  grid_trigger();
+  const long long row = blockIdx.x, slot = slot_mapping[row];
+  const int half = D >> 1, vecs = half >> 3, rot = (Hq + Hkv) * vecs, kv_width = Hkv * D;
+  const size_t table = static_cast<size_t>(pos[row]) * half;
+  __nv_bfloat16* r = qkv + row * row_stride;
+  for (int idx = threadIdx.x; idx < rot + (kv_width >> 3); idx += RC_THREADS) {
+    if (idx >= rot) {
+      const int v = idx - rot;
+      if (slot >= 0)
+        reinterpret_cast<uint4*>(v_cache + slot * kv_width)[v] = reinterpret_cast<const uint4*>(r + (Hq + Hkv) * D)[v];
+      continue;
+    }
+    const int head = idx / vecs, c = (idx - head * vecs) * 8;
+    __nv_bfloat16* base = r + head * D + c;
+    const uint4 a4 = *reinterpret_cast<const uint4*>(base), b4 = *reinterpret_cast<const uint4*>(base + half);
+    const uint32_t aw[4] = {a4.x, a4.y, a4.z, a4.w}, bw[4] = {b4.x, b4.y, b4.z, b4.w};
+    uint32_t oa[4], ob[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 cs = *reinterpret_cast<const float2*>(cos_t + table + c + 2 * e);
+      const float2 sn = *reinterpret_cast<const float2*>(sin_t + table + c + 2 * e);
+      const float2 a = unpack_bf16x2(aw[e]), b = unpack_bf16x2(bw[e]);
+      oa[e] = pack_bf16x2(a.x * cs.x - b.x * sn.x, a.y * cs.y - b.y * sn.y);
+      ob[e] = pack_bf16x2(b.x * cs.x + a.x * sn.x, b.y * cs.y + a.y * sn.y);
+    }
+    const uint4 ra = make_uint4(oa[0], oa[1], oa[2], oa[3]), rb = make_uint4(ob[0], ob[1], ob[2], ob[3]);
+    *reinterpret_cast<uint4*>(base) = ra;
+    *reinterpret_cast<uint4*>(base + half) = rb;
+    if (head >= Hq && slot >= 0) {
+      __nv_bfloat16* dst = k_cache + slot * kv_width + (head - Hq) * D + c;
+      *reinterpret_cast<uint4*>(dst) = ra;
+      *reinterpret_cast<uint4*>(dst + half) = rb;
+    }
+  }
+}
+
 // k_cache / v_cache: [num_blocks][block_size][Hkv][D] bf16.  slot = block * block_size + offset.
 __global__ void kv_cache_write_kernel(const __nv_bfloat16* __restrict__ qkv, int row_stride, int k_col0, int v_col0,
                                       __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache,
@@ -89,6 +134,8 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, const
   const int split = blockIdx.x, hk = blockIdx.y, seq = blockIdx.z;
   const int group = Hq / Hkv;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
+  grid_wait();
+  grid_trigger();
   const int len = seq_lens[seq];
   const int share = (max(chunk, (len + splits - 1) / splits) + 15) & ~15;
   const int t0 = split * share, t1 = min(len, t0 + share);
@@ -319,6 +366,17 @@ extern "C" int ts_kv_cache_write(const void* qkv, int row_stride, int k_col0, in
   return (int)cudaGetLastError();
 }
 
+// D a multiple of 16; rows of qkv (q | k | v heads) 16-byte aligned; cos / sin: fp32 [positions][D / 2]; slot < 0: not cached.
+extern "C" int ts_rope_cache(void* qkv, long long row_stride, const float* cos_t, const float* sin_t, const int* pos,
+                             const long long* slot_mapping, void* k_cache, void* v_cache, long long rows, int Hq, int Hkv, int D,
+                             void* stream) {
+  if (rows <= 0) return 0;
+  if (D <= 0 || D % 16 || row_stride % 8 || (reinterpret_cast<uintptr_t>(qkv) & 15u) || rows > 0x7fffffffll) return -10;
+  return launch_chained(rope_cache_kernel, dim3((unsigned)rows), dim3(RC_THREADS), 0, reinterpret_cast<cudaStream_t>(stream), 1,
+                        true, (__nv_bfloat16*)qkv, row_stride, cos_t, sin_t, pos, slot_mapping, (__nv_bfloat16*)k_cache,
+                        (__nv_bfloat16*)v_cache, Hq, Hkv, D);
+}
+
 extern "C" int ts_kv_gather(const void* k_cache, const void* v_cache, const int* block_table, int max_blocks,
                             const int* starts, const int* lens, int sequences, int max_len, int block_size, int kv_width,
                             void* out, void* stream) {
@@ -337,20 +395,10 @@ template <int D, bool CLUSTER>
 static int launch_decode(const void* q, int q_stride, const void* k_cache, const void* v_cache, const int* block_table,
                          int max_blocks, const int* seq_lens, void* out, int out_stride, float* part_out, float* part_lse,
                          int num_seqs, int Hq, int Hkv, int block_size, int chunk, int splits, float scale_log2, cudaStream_t st) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(splits, Hkv, num_seqs);
-  cfg.blockDim = dim3(DEC_WARPS * 32);
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = CLUSTER ? splits : 1;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return (int)cudaLaunchKernelEx(&cfg, decode_attention_kernel<D, CLUSTER>, (const __nv_bfloat16*)q, q_stride,
-                                 (const __nv_bfloat16*)k_cache, (const __nv_bfloat16*)v_cache, block_table, max_blocks, seq_lens,
-                                 (__nv_bfloat16*)out, out_stride, part_out, part_lse, Hq, Hkv, block_size, chunk, splits,
-                                 scale_log2);
+  return launch_chained(decode_attention_kernel<D, CLUSTER>, dim3(splits, Hkv, num_seqs), dim3(DEC_WARPS * 32), 0, st,
+                        CLUSTER ? splits : 1, true, (const __nv_bfloat16*)q, q_stride, (const __nv_bfloat16*)k_cache,
+                        (const __nv_bfloat16*)v_cache, block_table, max_blocks, seq_lens, (__nv_bfloat16*)out, out_stride, part_out,
+                        part_lse, Hq, Hkv, block_size, chunk, splits, scale_log2);
 }
 
 }  // namespace ts

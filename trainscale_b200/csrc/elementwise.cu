@@ -217,6 +217,44 @@ __global__ void __launch_bounds__(128) rmsnorm_fwd_warp_kernel(const __nv_bfloat
   }
 }
 
+// RMSNorm of the few rows of a serving step (the rows of rmsnorm_fwd_warp_kernel, one warp each, take 6.4 us of dependent loads
+// and shuffles whatever their number): one CTA per row, one 16-byte vector per thread, so a row costs one load latency; the
+// weight comes before the rows' producer has finished (chained launch).  2048 wide, 16 rows, back to back: 3.9 -> 1.9 us.
+__global__ void __launch_bounds__(1024) rmsnorm_step_kernel(const __nv_bfloat16* __restrict__ x,
+                                                            const __nv_bfloat16* __restrict__ residual,
+                                                            const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
+                                                            __nv_bfloat16* __restrict__ res_out, int H, float eps,
+                                                            float w_offset) {
+  __shared__ float scratch[32];
+  const size_t at = static_cast<size_t>(blockIdx.x) * H + threadIdx.x * 8;
+  const bool in = threadIdx.x * 8 < H;
+  float wv[8], a[8];
+  if (in) load8(w + threadIdx.x * 8, wv);
+  grid_wait();
+  grid_trigger();
+  float ss = 0.f;
+  if (in) {
+    load8(x + at, a);
+    if (residual) {
+      float b[8];
+      load8(residual + at, b);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) a[e] += b[e];
+      uint4 sum = pack_u4(a);            // rounded to bf16 as the stored stream is
+      *reinterpret_cast<uint4*>(res_out + at) = sum;
+      unpack_u4(sum, a);
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) ss += a[e] * a[e];
+  }
+  const float rstd = rsqrtf(block_sum(ss, scratch) / H + eps);
+  if (in) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) a[e] = a[e] * rstd * (wv[e] + w_offset);
+    store8(y + at, a);
+  }
+}
+
 // RMSNorm backward. Each CTA walks rows blockIdx.x, +gridDim.x, ... ; dx is written per row and the
 // weight gradient is accumulated in registers and written as one fp32 partial row per CTA
 // (dw_partial[gridDim.x][H]); rmsnorm_dw_reduce_kernel sums the partials. `dres` (optional) is an extra
@@ -942,6 +980,14 @@ extern "C" int ts_rmsnorm_fwd(const void* x, const void* residual, const void* w
   rmsnorm_fwd_kernel<<<(unsigned)rows, NORM_THREADS, 0, ST(stream)>>>(
       (const bf16*)x, (const bf16*)residual, (const bf16*)w, (bf16*)y, (bf16*)res_out, rstd, H, eps, w_offset);
   return (int)cudaGetLastError();
+}
+
+// The same for the rows of a serving step, H <= 8192: no rstd, chained launch (w is not written by the kernel before this one).
+extern "C" int ts_rmsnorm_step(const void* x, const void* residual, const void* w, void* y, void* res_out, long long rows, int H,
+                               float eps, float w_offset, void* stream) {
+  if (H % 8 != 0 || H <= 0 || H > 8192 || rows <= 0 || rows > 0x7fffffffll) return -10;
+  return launch_chained(rmsnorm_step_kernel, dim3((unsigned)rows), dim3((unsigned)((H / 8 + 31) / 32 * 32)), 0, ST(stream), 1, true,
+                        (const bf16*)x, (const bf16*)residual, (const bf16*)w, (bf16*)y, (bf16*)res_out, H, eps, w_offset);
 }
 
 // Number of fp32 partial rows the backward pass needs in `dw_partial` ([parts][H]).

@@ -88,6 +88,34 @@ inline int make_tmap_3d(CUtensorMap* out, const void* base, CUtensorMapDataType 
   return r == CUDA_SUCCESS ? 0 : -3;
 }
 
+// Launch in clusters of `cluster` CTAs along x; `chained`: the kernel may start before its predecessor in the stream has
+// finished (common.cuh grid_wait), which hides its launch, its set-up and the loads that do not depend on the predecessor.
+template <typename... P, typename... A>
+inline int launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cluster, bool chained,
+                          A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (cluster > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = static_cast<unsigned>(cluster);
+    attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  if (chained) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n].val.programmaticStreamSerializationAllowed = 1;
+    ++n;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = static_cast<unsigned>(n);
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+}
+
 inline int sm_count() {
   static int n = 0;
   if (n == 0) {

@@ -97,21 +97,33 @@ rows_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   const uint32_t tmem_base = tmem_slot;
   bool alive = true;
 
+  auto load_w = [&](int s, int kb) {
+    uint8_t* dst = smem + s * stage_bytes;
+    mbar_expect_tx(&full_bar[s], stage_bytes);
+    tma_load_2d(dst, &tmW, &full_bar[s], kb * 64, n0);
+    if (GLU) tma_load_2d(dst + RG_W_BYTES / 2, &tmW, &full_bar[s], kb * 64, p.N + n0);
+  };
+  auto load_x = [&](int s, int kb) {
+    tma_load_2d(smem + s * stage_bytes + RG_W_BYTES, &tmX, &full_bar[s], kb * 64, m0);
+  };
+  // the first weights come while the kernel that writes the rows may still be running
+  const int ahead = min(p.stages, kb1 - kb0);
+  const bool producer = warp == 0 && elect_one_sync();
+  if (producer)
+    for (int it = 0; it < ahead; ++it) load_w(it, kb0 + it);
+  __syncwarp();
+  grid_wait();
+  grid_trigger();
+
   if (warp == 0) {
-    if (elect_one_sync()) {
+    if (producer) {
       int it = 0;
-      for (int kb = kb0; kb < kb1; ++kb, ++it) {
+      for (; it < ahead; ++it) load_x(it, kb0 + it);
+      for (int kb = kb0 + ahead; kb < kb1; ++kb, ++it) {
         const int s = it % p.stages;
         if (!mbar_wait(&empty_bar[s], ((it / p.stages) & 1u) ^ 1u, alive, 100)) break;
-        mbar_expect_tx(&full_bar[s], stage_bytes);
-        uint8_t* dst = smem + s * stage_bytes;
-        if (GLU) {
-          tma_load_2d(dst, &tmW, &full_bar[s], kb * 64, n0);
-          tma_load_2d(dst + RG_W_BYTES / 2, &tmW, &full_bar[s], kb * 64, p.N + n0);
-        } else {
-          tma_load_2d(dst, &tmW, &full_bar[s], kb * 64, n0);
-        }
-        tma_load_2d(dst + RG_W_BYTES, &tmX, &full_bar[s], kb * 64, m0);
+        load_w(s, kb);
+        load_x(s, kb);
       }
       if (!alive) {
         // tear-down after a failed wait: give the loads that are still in flight a bounded time to land
@@ -230,26 +242,15 @@ static int rows_splits(int tiles, int k_blocks, int resident) {
 }
 
 template <int ACT>
-static int launch_rows(const CUtensorMap& tW, const CUtensorMap& tX, const RowsGemmParams& p, int tiles, size_t smem, cudaStream_t st) {
+static int launch_rows(const CUtensorMap& tW, const CUtensorMap& tX, const RowsGemmParams& p, int tiles, size_t smem, bool chained, cudaStream_t st) {
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(rows_gemm_kernel<ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, RG_RING + 1024);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(tiles * p.splits), (unsigned)((p.M + RG_TOKENS - 1) / RG_TOKENS));
-  cfg.blockDim = dim3(RG_THREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)p.splits;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return (int)cudaLaunchKernelEx(&cfg, rows_gemm_kernel<ACT>, tW, tX, p);
+  const dim3 grid((unsigned)(tiles * p.splits), (unsigned)((p.M + RG_TOKENS - 1) / RG_TOKENS));
+  return launch_chained(rows_gemm_kernel<ACT>, grid, dim3(RG_THREADS), smem, st, p.splits, chained, tW, tX, p);
 }
 
 }  // namespace ts
@@ -258,9 +259,10 @@ TS_DEFINE_ERROR_API(ts_rows_gemm)
 using namespace ts;
 
 // X [M][ldx], W [rows][ldw], out [M][ldo] (bf16, or fp32 with out_fp32).  glu < 0: W has N rows.  glu 0 silu, 1 gelu, 2 gelu in its
-// tanh form: W has 2 N rows, gates first, out = act(gate) * up.  Rows of X and W are 16-byte aligned.
+// tanh form: W has 2 N rows, gates first, out = act(gate) * up.  Rows of X and W are 16-byte aligned.  chained: see launch_chained;
+// the kernel before this one must not write W.
 extern "C" int ts_rows_gemm(const void* X, const void* W, void* out, int M, int N, int K, long long ldx, long long ldw,
-                            long long ldo, int out_fp32, int glu, void* stream) {
+                            long long ldo, int out_fp32, int glu, int chained, void* stream) {
   if (M <= 0 || N <= 0 || K <= 0 || glu > 2) return -10;
   RowsGemmParams p;
   p.M = M; p.N = N; p.K = K; p.out = out; p.ldo = ldo; p.out_fp32 = out_fp32;
@@ -285,8 +287,8 @@ extern "C" int ts_rows_gemm(const void* X, const void* W, void* out, int M, int 
   rc = make_tmap_2d(&tX, X, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)M, (uint64_t)K, (uint64_t)ldx, (uint32_t)p.mt, 64);
   if (rc) return rc * 100 - 2;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (glu < 0) return launch_rows<-1>(tW, tX, p, tiles, smem, st);
-  if (glu == 0) return launch_rows<0>(tW, tX, p, tiles, smem, st);
-  if (glu == 1) return launch_rows<1>(tW, tX, p, tiles, smem, st);
-  return launch_rows<2>(tW, tX, p, tiles, smem, st);
+  if (glu < 0) return launch_rows<-1>(tW, tX, p, tiles, smem, chained != 0, st);
+  if (glu == 0) return launch_rows<0>(tW, tX, p, tiles, smem, chained != 0, st);
+  if (glu == 1) return launch_rows<1>(tW, tX, p, tiles, smem, chained != 0, st);
+  return launch_rows<2>(tW, tX, p, tiles, smem, chained != 0, st);
 }

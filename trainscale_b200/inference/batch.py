@@ -174,6 +174,11 @@ class StepBatch:
         return self._contexts["portions"]
 
     @property
+    def all_wanted(self) -> bool:
+        """Logits of every row, in order, are asked for (a captured decode always does)."""
+        return self.host is None or self.host.out_rows == list(range(self.num_tokens))
+
+    @property
     def longest_single(self) -> int:
         """Upper bound of the keys that a single-token entry sees."""
         h = self.host

@@ -28,6 +28,7 @@ import torch
 from ..utils.refargs import ANY, reference_kwargs
 
 from ..core.types import Err, Ok, Result
+from ..models.llama import RMSNorm
 from ..ops import _lib, activation, attention, flash, gemm, norm, rope
 from .batch import HostBatch, StepBatch, StepEntry
 from .kv_cache import CacheSpec, PagedKVCache
@@ -287,12 +288,32 @@ class ModelRunner:
         return x
 
     def _lin(self, li: int, wname: str, w: torch.Tensor, x: torch.Tensor, adapter_ids) -> torch.Tensor:
-        y = gemm.step_linear(x, w)
+        y = gemm.step_linear(x, w, chained=True)      # no kernel of a step writes weights
         if self.lora is not None and adapter_ids is not None:
             d = self.lora.delta(li, wname, x, adapter_ids)
             if d is not None:
                 y = y + d
         return y
+
+    def _norm(self, module, x: torch.Tensor, res: torch.Tensor | None):
+        if self.cuda and type(module) is RMSNorm:
+            return norm.rmsnorm_step(x, module.weight, module.eps, res, module.offset)
+        return module(x, res)
+
+    def _rotate_and_cache(self, layer: int, qkv: torch.Tensor, batch: StepBatch) -> torch.Tensor:
+        """Projection rows with rotated queries and keys; keys and values go to the cache."""
+        c = self.cfg
+        if self.cuda and not c.rope_interleaved and c.head_dim % 16 == 0 and qkv.stride(1) == 1 and qkv.stride(0) % 8 == 0:
+            rc = _lib.load("decode").ts_rope_cache(
+                _lib.ptr(qkv), ctypes.c_longlong(qkv.stride(0)), _lib.ptr(self.cos), _lib.ptr(self.sin), _lib.ptr(batch.positions),
+                _lib.ptr(batch.slots), _lib.ptr(self.cache.k[layer]), _lib.ptr(self.cache.v[layer]),
+                ctypes.c_longlong(qkv.shape[0]), self.Hq, self.Hkv, c.head_dim, _lib.stream_ptr())
+            _lib.check(rc, "ts_rope_cache")
+            return qkv
+        qkv = rope.apply_rope_qkv(qkv.unsqueeze(0), self.Hq + self.Hkv, c.head_dim, self.cos, self.sin,
+                                  batch.positions.unsqueeze(0), qkv.shape[0], 0, c.rope_interleaved)[0]
+        self._write_cache(layer, qkv, batch.slots)
+        return qkv
 
     def _write_cache(self, layer: int, qkv2d: torch.Tensor, slots: torch.Tensor) -> None:
         c = self.cfg
@@ -380,7 +401,7 @@ class ModelRunner:
         """The decoder over a flattened token batch; returns the final-norm hidden state of the wanted rows."""
         if self.own_layers:
             return self.model.serve(batch, self.cache)
-        pos32, adapter_ids = batch.positions, batch.adapter_ids
+        adapter_ids = batch.adapter_ids
         m, c = self.model.model, self.cfg
         x = m.embed_tokens(batch.token_ids)
         if getattr(c, "scale_embeddings", False):
@@ -388,26 +409,24 @@ class ModelRunner:
         res = None
         for li, layer in enumerate(m.layers):
             attn, mlp = getattr(layer.self_attn, "inner", layer.self_attn), getattr(layer.mlp, "inner", layer.mlp)
-            h, res = layer.input_layernorm(x, res)
+            h, res = self._norm(layer.input_layernorm, x, res)
             qkv = self._lin(li, "wqkv", attn.wqkv, h, adapter_ids)
             if attn.bqkv is not None:
                 qkv = qkv + attn.bqkv
-            qkv = rope.apply_rope_qkv(qkv.unsqueeze(0), self.Hq + self.Hkv, c.head_dim, self.cos, self.sin,
-                                      pos32.unsqueeze(0), qkv.shape[0], 0, c.rope_interleaved)[0]
-            self._write_cache(li, qkv, batch.slots)
+            qkv = self._rotate_and_cache(li, qkv, batch)
             a = self._attend(li, qkv, batch)
             a = self._reduce(self._lin(li, "wo", attn.wo, a, adapter_ids))
-            h, res = layer.post_attention_layernorm(a, res)
+            h, res = self._norm(layer.post_attention_layernorm, a, res)
             if hasattr(mlp, "router"):            # mixture of experts: the block routes by itself
                 x = layer.mlp(h)
             else:
                 if self.lora is not None and adapter_ids is not None:
                     h = activation.glu(self._lin(li, "w_gate_up", mlp.w_gate_up, h, adapter_ids), mlp.act)
                 else:
-                    h = gemm.step_glu(h, mlp.w_gate_up, mlp.act)
+                    h = gemm.step_glu(h, mlp.w_gate_up, mlp.act, chained=True)
                 x = self._reduce(self._lin(li, "w_down", mlp.w_down, h, adapter_ids))
-        x, _ = m.norm(x, res)
-        return x[batch.out_rows]
+        x, _ = self._norm(m.norm, x, res)
+        return x if batch.all_wanted else x[batch.out_rows]
 
     @torch.no_grad()
     def forward(self, batch: StepBatch) -> torch.Tensor:
@@ -491,7 +510,7 @@ class ModelRunner:
         """fp32 logits of hidden states [n, H]."""
         if self.own_layers or self.tp is not None or not self.cuda:
             return self.model.logits(hidden).float()
-        z, cap = gemm.step_linear(hidden, self.model.head_weight, torch.float32), self.cfg.final_logit_softcap
+        z, cap = gemm.step_linear(hidden, self.model.head_weight, torch.float32, chained=True), self.cfg.final_logit_softcap
         return cap * torch.tanh(z / cap) if cap and cap > 0 else z
 
 

@@ -220,20 +220,22 @@ def _streamed(x: torch.Tensor, w: torch.Tensor) -> bool:
     return M <= 32 or N <= 12288 and (M <= 128 or M <= 256 and K >= 3 * N)
 
 
-def _stream_rows(x: torch.Tensor, w: torch.Tensor, cols: int, out_dtype: torch.dtype, glu: int) -> torch.Tensor:
+def _stream_rows(x: torch.Tensor, w: torch.Tensor, cols: int, out_dtype: torch.dtype, glu: int,
+                 chained: bool = False) -> torch.Tensor:
     out = torch.empty(x.shape[0], cols, dtype=out_dtype, device=x.device)
     rc = _lib.load("rows_gemm").ts_rows_gemm(
         _lib.ptr(x), _lib.ptr(w), _lib.ptr(out), x.shape[0], cols, x.shape[1], _c.c_longlong(x.stride(0)),
-        _c.c_longlong(w.stride(0)), _c.c_longlong(cols), int(out_dtype == torch.float32), glu, _lib.stream_ptr())
+        _c.c_longlong(w.stride(0)), _c.c_longlong(cols), int(out_dtype == torch.float32), glu, int(chained), _lib.stream_ptr())
     _lib.check(rc, "ts_rows_gemm")
     return out
 
 
 @torch.no_grad()
-def step_linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = None) -> torch.Tensor:
-    """x [M, K] @ w [N, K]^T of a serving step, optionally with an fp32 result."""
+def step_linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = None, chained: bool = False) -> torch.Tensor:
+    """x [M, K] @ w [N, K]^T of a serving step, optionally with an fp32 result.  `chained`: the weights may be fetched while
+    the kernel before this one still runs, so that one must not be what writes `w`."""
     if _streamed(x, w):
-        return _stream_rows(x, w, w.shape[0], out_dtype or x.dtype, -1)
+        return _stream_rows(x, w, w.shape[0], out_dtype or x.dtype, -1, chained)
     if out_dtype is not None and x.is_cuda and x.dtype == w.dtype == torch.bfloat16 and x.numel():
         return matmul_nt(x, w, out_dtype=out_dtype).view(*x.shape[:-1], w.shape[0])
     y = linear(x, w)
@@ -241,10 +243,10 @@ def step_linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None 
 
 
 @torch.no_grad()
-def step_glu(x: torch.Tensor, w: torch.Tensor, act: str) -> torch.Tensor:
-    """act(x @ gate^T) * (x @ up^T) of a serving step; w [2 I, K] = gate | up."""
+def step_glu(x: torch.Tensor, w: torch.Tensor, act: str, chained: bool = False) -> torch.Tensor:
+    """act(x @ gate^T) * (x @ up^T) of a serving step; w [2 I, K] = gate | up; `chained` as in `step_linear`."""
     if _streamed(x, w) and w.shape[0] % 2 == 0:
-        return _stream_rows(x, w, w.shape[0] // 2, x.dtype, activation._ACT[act])
+        return _stream_rows(x, w, w.shape[0] // 2, x.dtype, activation._ACT[act], chained)
     return activation.glu(linear(x, w), act)
 
 

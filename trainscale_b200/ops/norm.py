@@ -100,6 +100,26 @@ def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float = 1e-5, residual: torch
     return rmsnorm_reference(x, w, eps, residual, w_offset)
 
 
+STEP_ROWS = 1024     # rows up to which a CTA per row (ts_rmsnorm_step) is taken; the warps of the other kernel then fill the GPU
+
+
+@torch.no_grad()
+def rmsnorm_step(x: torch.Tensor, w: torch.Tensor, eps: float, residual: torch.Tensor | None = None, w_offset: float = 0.0):
+    """`rmsnorm` of the rows of a serving step, without autograd."""
+    H = x.shape[-1]
+    if not (x.is_cuda and x.dtype == w.dtype == torch.bfloat16 and H % 8 == 0 and H <= 8192 and x.dim() == 2
+            and 0 < x.shape[0] <= STEP_ROWS and (residual is None or residual.shape == x.shape and residual.dtype == x.dtype)
+            and all(t is None or t.is_contiguous() and t.data_ptr() % 16 == 0 for t in (x, w, residual))):
+        return rmsnorm(x, w, eps, residual, w_offset)
+    y = torch.empty_like(x)
+    res = x if residual is None else torch.empty_like(x)
+    rc = _lib.load("elementwise").ts_rmsnorm_step(
+        _lib.ptr(x), _lib.ptr(residual), _lib.ptr(w), _lib.ptr(y), _lib.ptr(None if residual is None else res),
+        ctypes.c_longlong(x.shape[0]), H, ctypes.c_float(eps), ctypes.c_float(w_offset), _lib.stream_ptr())
+    _lib.check(rc, "ts_rmsnorm_step")
+    return y, res
+
+
 class _LayerNormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, b, eps):
