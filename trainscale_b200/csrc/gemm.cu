@@ -6,8 +6,11 @@
 //   warp 1      MMA issuer     - one elected thread issues tcgen05.mma (128 x BN x 16) into one of two TMEM
 //                                accumulators, tcgen05.commit releases ring slots / publishes the accumulator
 //   warps 2..5  epilogue       - tcgen05.ld the finished accumulator (each warp owns its 32 TMEM lanes),
-//                                scale / add / convert and store with 16-byte vector stores, while the MMA
-//                                warp already works on the next tile in the other accumulator
+//                                scale / convert, while the MMA warp already works on the next tile in the other
+//                                accumulator.  bf16 results leave through shared memory by TMA (32 rows x 64 columns per
+//                                store): a warp's direct 16-byte stores touch 32 rows each, 4000 cycles of the load/store
+//                                unit for a 128 x 256 tile, which short reductions cannot hide.  Direct stores remain for
+//                                results that are added to C, fp32, gated products and rows TMA cannot address
 // Operands may be K-major or MN-major in memory, so forward (X W^T), dgrad (dY W) and wgrad (dY^T X)
 // all run without a transpose pass.
 //
@@ -44,7 +47,10 @@ struct GemmParams {
   int act;                  // epilogue activation of common.cuh product_act or glu_act (modes 0 and 1; 0: none)
   float act_a, act_b;       // its constants
   int act_cols;             // columns it applies to, from the first; a multiple of 32 unless all
+  int tma_c;                // results leave by TMA
 };
+
+constexpr int GEMM_EP_BYTES = 4 * 2 * 4096;   // two 32-row x 64-column staging tiles per epilogue warp
 
 // 32 accumulator columns of a gated product = 16 gates and the 16 factors of the same outputs: 16 results.
 __device__ __forceinline__ void gemm_store_glu(const GemmParams& p, const uint32_t* r, size_t row, int col0) {
@@ -153,6 +159,45 @@ __device__ __forceinline__ void gemm_store_chunk(const GemmParams& p, const uint
   }
 }
 
+// COLS accumulator columns of the warp's 32 rows (C row `row0` on), by TMA from the warp's two staging tiles.  `issued` counts the
+// warp's stores: a tile is reused when the store before the last has read it.
+template <int COLS>
+__device__ __forceinline__ void gemm_store_tma(const GemmParams& p, const CUtensorMap* tmC, uint32_t t_row, uint8_t* stage,
+                                               int row0, int n0, uint32_t& issued) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll 1
+  for (int c = 0; c < COLS / 64; ++c) {
+    const int col0 = n0 + c * 64;
+    if (col0 >= p.N) break;
+    uint32_t r[64];
+    tmem_ld_32x32b_x32(t_row + c * 64, r);
+    tmem_ld_32x32b_x32(t_row + c * 64 + 32, r + 32);
+    tc_wait_ld();
+    if (p.act != 0) {
+      gemm_activate(p, r, col0);
+      gemm_activate(p, r + 32, col0 + 32);
+    }
+    uint8_t* buf = stage + (issued & 1u) * 4096;
+    if (lane == 0) tma_store_wait_read<1>();
+    __syncwarp();
+#pragma unroll
+    for (int ch = 0; ch < 8; ++ch) {
+      uint32_t o[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        o[e] = pack_bf16x2(__uint_as_float(r[8 * ch + 2 * e]) * p.alpha, __uint_as_float(r[8 * ch + 2 * e + 1]) * p.alpha);
+      *reinterpret_cast<uint4*>(buf + sw128_offset(lane, ch)) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+      tma_store_2d(tmC, buf, col0, row0);
+      tma_store_commit();
+    }
+    ++issued;
+  }
+}
+
 struct GemmTile {
   int m0, n0;        // tile origin in the A-row / B-row (output) index spaces
   int b_off;         // MODE 1: offset of this tile's expert along B's row (K-major) or K (MN-major) coordinate
@@ -167,7 +212,7 @@ struct GemmSmem {
   static constexpr int B_BYTES = BN * GEMM_BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int BAR_BYTES = 256;
-  static constexpr int TOTAL = STAGES * STAGE_BYTES + BAR_BYTES + 1024;   // + alignment slack
+  static constexpr int TOTAL = STAGES * STAGE_BYTES + GEMM_EP_BYTES + BAR_BYTES + 1024;   // + alignment slack
 };
 
 // MODE 0: dense.  MODE 1: grouped rows - every 128-row tile of A/C belongs to one expert whose weight is a slab of
@@ -175,7 +220,8 @@ struct GemmSmem {
 // buffer).  MODE 2: grouped reduction - one output slab per expert, reduced over that expert's row segment (wgrad).
 template <int BN, int MODE>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
-gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmParams p) {
+gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                 const __grid_constant__ CUtensorMap tmC, GemmParams p) {
   using S = GemmSmem<BN>;
   constexpr int STAGES = S::STAGES;
   constexpr uint32_t TMEM_COLS = (2 * BN <= 32) ? 32 : 2 * BN;   // two accumulators
@@ -184,7 +230,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* smem_a = smem;
   uint8_t* smem_b = smem + STAGES * S::A_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * S::STAGE_BYTES);
+  uint8_t* smem_c = smem + STAGES * S::STAGE_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_c + GEMM_EP_BYTES);
   uint64_t* full_bar = bars;                    // [STAGES]
   uint64_t* empty_bar = bars + STAGES;          // [STAGES]
   uint64_t* tfull_bar = bars + 2 * STAGES;      // [2]
@@ -332,7 +379,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   } else {
     // ------------------------------ epilogue (warps 2..5) ------------------------------
     const int q = warp & 3;   // TMEM lane quarter this warp may access
-    uint32_t tile_it = 0;
+    uint32_t tile_it = 0, issued = 0;
     for (int t = blockIdx.x; t < num_tiles && alive; t += gridDim.x) {
       GemmTile ti;
       if (!tile_info(t, ti)) continue;
@@ -355,23 +402,29 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       if (!mbar_wait(&tfull_bar[acc], acc_ph, alive, 300)) break;
       tc_fence_after_sync();
       const uint32_t t_row = tmem_base + acc * BN + (static_cast<uint32_t>(q * 32) << 16);
+      if (p.tma_c) {
+        if (m0 + q * 32 < p.M)
+          gemm_store_tma<BN>(p, &tmC, t_row, smem_c + q * 8192, static_cast<int>(ti.c_row0) + m0 + q * 32, n0, issued);
+      } else {
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32b_x32(t_row + c * 32, r);
-        tc_wait_ld();
-        const int col0 = n0 + c * 32;
-        if (MODE != 2 && p.act >= ACT_FIRST_GLU) {
-          if (row < p.M && col0 < p.N) gemm_store_glu(p, r, ti.c_row0 + row, col0);
-          continue;
+        for (int c = 0; c < BN / 32; ++c) {
+          uint32_t r[32];
+          tmem_ld_32x32b_x32(t_row + c * 32, r);
+          tc_wait_ld();
+          const int col0 = n0 + c * 32;
+          if (MODE != 2 && p.act >= ACT_FIRST_GLU) {
+            if (row < p.M && col0 < p.N) gemm_store_glu(p, r, ti.c_row0 + row, col0);
+            continue;
+          }
+          if (MODE != 2 && p.act != 0) gemm_activate(p, r, col0);
+          if (row < p.M && col0 < p.N) gemm_store_chunk(p, r, ti.c_row0 + row, col0);
         }
-        if (MODE != 2 && p.act != 0) gemm_activate(p, r, col0);
-        if (row < p.M && col0 < p.N) gemm_store_chunk(p, r, ti.c_row0 + row, col0);
       }
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty_bar[acc]);
     }
+    if (lane == 0 && issued) tma_store_wait<0>();
   }
 
   tc_fence_before_sync();
@@ -391,10 +444,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 // ---------------------------------------------------------------------------------------------------------
 constexpr int G2_STAGES = 6;
 constexpr int G2_STAGE_BYTES = 32768;      // A 128x64 + B-half 128x64, bf16
-constexpr int G2_SMEM = G2_STAGES * G2_STAGE_BYTES + 256 + 1024;
+constexpr int G2_SMEM = G2_STAGES * G2_STAGE_BYTES + GEMM_EP_BYTES + 256 + 1024;
 
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
-gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmParams p) {
+gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                      const __grid_constant__ CUtensorMap tmC, GemmParams p) {
   constexpr int STAGES = G2_STAGES;
   constexpr int BN = 256;
   constexpr uint32_t TMEM_COLS = 512;
@@ -403,7 +457,8 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* smem_a = smem;
   uint8_t* smem_b = smem + STAGES * 16384;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * G2_STAGE_BYTES);
+  uint8_t* smem_c = smem + STAGES * G2_STAGE_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_c + GEMM_EP_BYTES);
   uint64_t* full_bar = bars;
   uint64_t* empty_bar = bars + STAGES;
   uint64_t* tfull_bar = bars + 2 * STAGES;
@@ -513,7 +568,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     }
   } else {
     const int q = warp & 3;
-    uint32_t tile_it = 0;
+    uint32_t tile_it = 0, issued = 0;
     for (int t = cluster_id; t < num_tiles && alive; t += num_clusters, ++tile_it) {
       int m0, n0;
       tile_coords(t, m0, n0);
@@ -522,23 +577,28 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       tc_fence_after_sync();
       const int row = m0 + q * 32 + lane;
       const uint32_t t_row = tmem_base + acc * BN + (static_cast<uint32_t>(q * 32) << 16);
+      if (p.tma_c) {
+        if (m0 + q * 32 < p.M) gemm_store_tma<BN>(p, &tmC, t_row, smem_c + q * 8192, m0 + q * 32, n0, issued);
+      } else {
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32b_x32(t_row + c * 32, r);
-        tc_wait_ld();
-        const int col0 = n0 + c * 32;
-        if (p.act >= ACT_FIRST_GLU) {
-          if (row < p.M && col0 < p.N) gemm_store_glu(p, r, static_cast<size_t>(row), col0);
-          continue;
+        for (int c = 0; c < BN / 32; ++c) {
+          uint32_t r[32];
+          tmem_ld_32x32b_x32(t_row + c * 32, r);
+          tc_wait_ld();
+          const int col0 = n0 + c * 32;
+          if (p.act >= ACT_FIRST_GLU) {
+            if (row < p.M && col0 < p.N) gemm_store_glu(p, r, static_cast<size_t>(row), col0);
+            continue;
+          }
+          if (p.act != 0) gemm_activate(p, r, col0);
+          if (row < p.M && col0 < p.N) gemm_store_chunk(p, r, static_cast<size_t>(row), col0);
         }
-        if (p.act != 0) gemm_activate(p, r, col0);
-        if (row < p.M && col0 < p.N) gemm_store_chunk(p, r, static_cast<size_t>(row), col0);
       }
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(&tempty_bar[acc], 0);   // the leader's MMA thread owns the accumulators
     }
+    if (lane == 0 && issued) tma_store_wait<0>();
   }
 
   tc_fence_before_sync();
@@ -550,7 +610,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   }
 }
 
-static int launch_gemm_2cta(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, cudaStream_t stream) {
+static int launch_gemm_2cta(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const GemmParams& p, cudaStream_t stream) {
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(gemm_bf16_2cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM);
@@ -572,11 +632,11 @@ static int launch_gemm_2cta(const CUtensorMap& tmA, const CUtensorMap& tmB, cons
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return (int)cudaLaunchKernelEx(&cfg, gemm_bf16_2cta_kernel, tmA, tmB, p);
+  return (int)cudaLaunchKernelEx(&cfg, gemm_bf16_2cta_kernel, tmA, tmB, tmC, p);
 }
 
 template <int BN, int MODE = 0>
-static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, cudaStream_t stream) {
+static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const GemmParams& p, cudaStream_t stream) {
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<BN, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -586,7 +646,7 @@ static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const Gem
   }
   const int tiles = p.num_m_tiles * p.num_n_tiles * (MODE == 2 ? p.num_groups : 1);
   const int grid = tiles < sm_count() ? tiles : sm_count();
-  gemm_bf16_kernel<BN, MODE><<<grid, GEMM_THREADS, GemmSmem<BN>::TOTAL, stream>>>(tmA, tmB, p);
+  gemm_bf16_kernel<BN, MODE><<<grid, GEMM_THREADS, GemmSmem<BN>::TOTAL, stream>>>(tmA, tmB, tmC, p);
   return (int)cudaGetLastError();
 }
 
@@ -594,6 +654,19 @@ static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const Gem
 static bool glu_ok(int act, const void* C, int N, int ldc, int out_fp32) {
   return act < ACT_FIRST_GLU || (N % (2 * GLU_BLOCK) == 0 && !out_fp32 && ldc % 8 == 0 && ldc >= N / 2 &&
                                  (reinterpret_cast<uintptr_t>(C) & 15u) == 0);
+}
+// Map of a bf16 result that TMA can store: p.tma_c and true, or direct stores (`tmC` is then unused).  The debug build checks every
+// store against C's extent, so it keeps the direct ones.  Slabs of a grouped reduction must end on a tile's border.
+static void plan_result(CUtensorMap& tmC, const CUtensorMap& unused, GemmParams& p, int slabs) {
+  tmC = unused;
+  p.tma_c = 0;
+#ifndef TS_DEBUG
+  if (p.out_fp32 || p.accumulate || p.act >= ACT_FIRST_GLU || (slabs > 1 && p.M % GEMM_BM) || p.ldc % 8 ||
+      (reinterpret_cast<uintptr_t>(p.C) & 15u) || p.ldc < p.N)
+    return;
+  p.tma_c = make_tmap_2d(&tmC, p.C, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)slabs * p.M, (uint64_t)p.N, (uint64_t)p.ldc, 32,
+                         64) == 0;
+#endif
 }
 static int result_cols(int act, int N) { return act >= ACT_FIRST_GLU ? N / 2 : N; }
 
@@ -658,11 +731,13 @@ extern "C" int ts_gemm_bf16_act(const void* A, const void* B, void* C, int M, in
     if (cut > 0 && cut < M) p.c_bytes = (static_cast<size_t>(M - cut - 1) * ldc + N) * (out_fp32 ? 4 : 2);
   }
 #endif
+  CUtensorMap tmC;
+  plan_result(tmC, tmA, p, 1);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (two_cta) return launch_gemm_2cta(tmA, tmB, p, st);
-  if (bn == 256) return launch_gemm<256>(tmA, tmB, p, st);
-  if (bn == 128) return launch_gemm<128>(tmA, tmB, p, st);
-  return launch_gemm<64>(tmA, tmB, p, st);
+  if (two_cta) return launch_gemm_2cta(tmA, tmB, tmC, p, st);
+  if (bn == 256) return launch_gemm<256>(tmA, tmB, tmC, p, st);
+  if (bn == 128) return launch_gemm<128>(tmA, tmB, tmC, p, st);
+  return launch_gemm<64>(tmA, tmB, tmC, p, st);
 }
 
 extern "C" int ts_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
@@ -718,15 +793,17 @@ extern "C" int ts_gemm_grouped_bf16_act(const void* A, const void* B, void* C, i
   p.act = act; p.act_a = p.act_b = 0.f; p.act_cols = N;
   p.c_bytes = (static_cast<size_t>((mode == 2 ? num_groups : 1)) * M - 1) * ldc * (out_fp32 ? 4 : 2) +
               static_cast<size_t>(result_cols(act, N)) * (out_fp32 ? 4 : 2);
+  CUtensorMap tmC;
+  plan_result(tmC, tmA, p, mode == 2 ? num_groups : 1);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (mode == 1) {
-    if (bn == 256) return launch_gemm<256, 1>(tmA, tmB, p, st);
-    if (bn == 128) return launch_gemm<128, 1>(tmA, tmB, p, st);
-    return launch_gemm<64, 1>(tmA, tmB, p, st);
+    if (bn == 256) return launch_gemm<256, 1>(tmA, tmB, tmC, p, st);
+    if (bn == 128) return launch_gemm<128, 1>(tmA, tmB, tmC, p, st);
+    return launch_gemm<64, 1>(tmA, tmB, tmC, p, st);
   }
-  if (bn == 256) return launch_gemm<256, 2>(tmA, tmB, p, st);
-  if (bn == 128) return launch_gemm<128, 2>(tmA, tmB, p, st);
-  return launch_gemm<64, 2>(tmA, tmB, p, st);
+  if (bn == 256) return launch_gemm<256, 2>(tmA, tmB, tmC, p, st);
+  if (bn == 128) return launch_gemm<128, 2>(tmA, tmB, tmC, p, st);
+  return launch_gemm<64, 2>(tmA, tmB, tmC, p, st);
 }
 
 extern "C" int ts_gemm_grouped_bf16(const void* A, const void* B, void* C, int mode, int M, int N, int K, int lda,
