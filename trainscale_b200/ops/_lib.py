@@ -47,7 +47,8 @@ def prepare(names: list[str]) -> None:
 
 
 def stream_ptr() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    # (the raw handle: a stream object costs 8 us of host time, at every launch)
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def ptr(t: torch.Tensor | None) -> ctypes.c_void_p:
@@ -55,7 +56,7 @@ def ptr(t: torch.Tensor | None) -> ctypes.c_void_p:
     that lives on another GPU is refused here, on the host, instead of faulting on the device."""
     if t is None:
         return ctypes.c_void_p(0)
-    if t.is_cuda and t.device.index != torch.cuda.current_device():
+    if t.is_cuda and t.get_device() != torch._C._cuda_getDevice():
         raise KernelError(f"tensor on {t.device} passed to a kernel while the current device is "
                           f"cuda:{torch.cuda.current_device()}; call torch.cuda.set_device (or use torch.cuda.device) first")
     return ctypes.c_void_p(t.data_ptr())

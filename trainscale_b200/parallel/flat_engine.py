@@ -829,7 +829,7 @@ class FlatShardedEngine:
             self._symm.check_status()
         if self.is_cuda:
             from ..ops import _lib
-            _lib.raise_on_any_device_error()
+            _lib.raise_on_loaded_device_error()      # (a library this process has not loaded has run no kernel)
 
     def _replicated_slices(self) -> list:
         """(unit, start, end) ranges of this rank's gradient shard that belong to `replicated_params`."""
