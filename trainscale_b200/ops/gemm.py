@@ -209,7 +209,8 @@ class _SplitLinearCPU(torch.autograd.Function):
 
 def _streamed(x: torch.Tensor, w: torch.Tensor) -> bool:
     """Whether weight tiles (csrc/rows_gemm.cu) beat 128-row token tiles.  Measured in us, streamed / token tiles, weights not in
-    L2.  Up to 32 rows always: 8 rows 7.6 / 11.5 (3072 x 2048), 83 / 108 (128256 x 2048); 32 rows 42 / 46 (28672 x 4096).  Up to
+    L2.  Up to 64 rows always: 8 rows 7.6 / 11.5 (3072 x 2048), 83 / 108 (128256 x 2048); 32 rows 42 / 46 (28672 x 4096); norm, gated
+    product and the product after it, 64 rows, chained 32 / 35 (2 x 8192 x 2048) and 74 / 80 (2 x 14336 x 4096), 96 rows equal.  Up to
     128 where token tiles are too few for the GPU: 128 rows 17.0 / 31.8 (2048 x 8192), 18.2 / 20.3 (6144 x 4096), but
     20.9 / 15.6 (16384 x 2048).  Beyond, every 128 rows read the weights again (from L2), which pays for a deep reduction:
     256 rows 18.9 / 31.7 (2048 x 8192), but 23.7 / 20.2 (6144 x 4096)."""
@@ -217,7 +218,7 @@ def _streamed(x: torch.Tensor, w: torch.Tensor) -> bool:
             and all(t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (x, w))):
         return False
     M, (N, K) = x.shape[0], w.shape
-    return M <= 32 or N <= 12288 and (M <= 128 or M <= 256 and K >= 3 * N)
+    return M <= 64 or N <= 12288 and (M <= 128 or M <= 256 and K >= 3 * N)
 
 
 def _stream_rows(x: torch.Tensor, w: torch.Tensor, cols: int, out_dtype: torch.dtype, glu: int,
