@@ -214,10 +214,12 @@ __device__ __forceinline__ float block_max(float v, float* scratch) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// chained launches (host_common.h launch_chained): the kernel may start while its predecessor in the stream still runs.  Every
-// thread calls grid_wait before it touches anything an earlier kernel may have written or may still read, and grid_trigger only
-// after it, so that a kernel that starts early finds everything BEFORE its predecessor finished and visible: weights, which no
-// kernel of a step writes, can be fetched ahead of grid_wait.  Both do nothing in an ordinary launch.
+// chained launches (host_common.h launch_chained): the kernel may start while its predecessors in the stream still run.  Every
+// thread calls grid_wait before it touches anything an earlier kernel may have written or may still read; it returns when the
+// predecessor has finished, which has itself waited for its own.  grid_trigger lets the next kernel of the chain start; it comes
+// first, but AFTER a block has its TMEM: blocks of the next kernel that took the columns first would wait for this one, and this
+// one for the columns.  Weights can be fetched ahead of grid_wait where no chained kernel and not the last ordinary kernel before
+// the chain writes them: that one had to wait for everything before it.  Both do nothing in an ordinary launch.
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

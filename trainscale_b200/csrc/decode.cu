@@ -16,8 +16,8 @@ __global__ void __launch_bounds__(RC_THREADS)
 rope_cache_kernel(__nv_bfloat16* __restrict__ qkv, long long row_stride, const float* __restrict__ cos_t,
                   const float* __restrict__ sin_t, const int* __restrict__ pos, const long long* __restrict__ slot_mapping,
                   __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache, int Hq, int Hkv, int D) {
-  grid_wait();
   grid_trigger();
+  grid_wait();
   const long long row = blockIdx.x, slot = slot_mapping[row];
   const int half = D >> 1, vecs = half >> 3, rot = (Hq + Hkv) * vecs, kv_width = Hkv * D;
   const size_t table = static_cast<size_t>(pos[row]) * half;
@@ -134,8 +134,8 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, const
   const int split = blockIdx.x, hk = blockIdx.y, seq = blockIdx.z;
   const int group = Hq / Hkv;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
-  grid_wait();
   grid_trigger();
+  grid_wait();
   const int len = seq_lens[seq];
   const int share = (max(chunk, (len + splits - 1) / splits) + 15) & ~15;
   const int t0 = split * share, t1 = min(len, t0 + share);

@@ -229,9 +229,9 @@ __global__ void __launch_bounds__(1024) rmsnorm_step_kernel(const __nv_bfloat16*
   const size_t at = static_cast<size_t>(blockIdx.x) * H + threadIdx.x * 8;
   const bool in = threadIdx.x * 8 < H;
   float wv[8], a[8];
+  grid_trigger();
   if (in) load8(w + threadIdx.x * 8, wv);
   grid_wait();
-  grid_trigger();
   float ss = 0.f;
   if (in) {
     load8(x + at, a);
@@ -982,7 +982,7 @@ extern "C" int ts_rmsnorm_fwd(const void* x, const void* residual, const void* w
   return (int)cudaGetLastError();
 }
 
-// The same for the rows of a serving step, H <= 8192: no rstd, chained launch (w is not written by the kernel before this one).
+// The same for the rows of a serving step, H <= 8192: no rstd, chained launch (w as the weights of launch_chained).
 extern "C" int ts_rmsnorm_step(const void* x, const void* residual, const void* w, void* y, void* res_out, long long rows, int H,
                                float eps, float w_offset, void* stream) {
   if (H % 8 != 0 || H <= 0 || H > 8192 || rows <= 0 || rows > 0x7fffffffll) return -10;

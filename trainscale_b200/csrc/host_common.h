@@ -89,7 +89,8 @@ inline int make_tmap_3d(CUtensorMap* out, const void* base, CUtensorMapDataType 
 }
 
 // Launch in clusters of `cluster` CTAs along x; `chained`: the kernel may start before its predecessor in the stream has
-// finished (common.cuh grid_wait), which hides its launch, its set-up and the loads that do not depend on the predecessor.
+// finished (common.cuh grid_wait), which hides its launch, its set-up and the loads that do not depend on the predecessors
+// (weights: see grid_wait for who may not write them).
 template <typename... P, typename... A>
 inline int launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cluster, bool chained,
                           A&&... args) {

@@ -106,14 +106,14 @@ rows_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   auto load_x = [&](int s, int kb) {
     tma_load_2d(smem + s * stage_bytes + RG_W_BYTES, &tmX, &full_bar[s], kb * 64, m0);
   };
-  // the first weights come while the kernel that writes the rows may still be running
+  grid_trigger();                    // (this block has its TMEM)
+  // the first weights come while the kernels before may still be running
   const int ahead = min(p.stages, kb1 - kb0);
   const bool producer = warp == 0 && elect_one_sync();
   if (producer)
     for (int it = 0; it < ahead; ++it) load_w(it, kb0 + it);
   __syncwarp();
   grid_wait();
-  grid_trigger();
 
   if (warp == 0) {
     if (producer) {
@@ -260,7 +260,7 @@ using namespace ts;
 
 // X [M][ldx], W [rows][ldw], out [M][ldo] (bf16, or fp32 with out_fp32).  glu < 0: W has N rows.  glu 0 silu, 1 gelu, 2 gelu in its
 // tanh form: W has 2 N rows, gates first, out = act(gate) * up.  Rows of X and W are 16-byte aligned.  chained: see launch_chained;
-// the kernel before this one must not write W.
+// no chained kernel and not the last ordinary one before them may write W.
 extern "C" int ts_rows_gemm(const void* X, const void* W, void* out, int M, int N, int K, long long ldx, long long ldw,
                             long long ldo, int out_fp32, int glu, int chained, void* stream) {
   if (M <= 0 || N <= 0 || K <= 0 || glu > 2) return -10;

@@ -234,7 +234,7 @@ def _stream_rows(x: torch.Tensor, w: torch.Tensor, cols: int, out_dtype: torch.d
 @torch.no_grad()
 def step_linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = None, chained: bool = False) -> torch.Tensor:
     """x [M, K] @ w [N, K]^T of a serving step, optionally with an fp32 result.  `chained`: the weights may be fetched while
-    the kernel before this one still runs, so that one must not be what writes `w`."""
+    the kernels before this one still run, back to the last ordinary launch, so none of these may be what writes `w`."""
     if _streamed(x, w):
         return _stream_rows(x, w, w.shape[0], out_dtype or x.dtype, -1, chained)
     if out_dtype is not None and x.is_cuda and x.dtype == w.dtype == torch.bfloat16 and x.numel():
