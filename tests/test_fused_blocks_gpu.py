@@ -79,3 +79,32 @@ def test_decoder_layer_op_selective_equals_plain_path():
     for n, p in m.named_parameters():
         d = (p.grad.float() - g0[n].float()).abs().max().item()
         assert d <= 2e-2 * max(g0[n].float().abs().max().item(), 1e-3), n
+
+
+# one vector per row, rows whose vectors are no multiple of a block, both sides of the unrolled loop's remainder
+@pytest.mark.parametrize("rows,I", [(1, 8), (3, 24), (257, 1376), (300, 2048)])
+@pytest.mark.parametrize("act", [0, 1, 2])
+def test_product_and_gradient_in_one_pass(rows, I, act):
+    """The bits of the two separate kernels."""
+    from trainscale_b200.ops import activation
+    torch.manual_seed(0)
+    gu, d = torch.randn(rows, 2 * I, device="cuda").bfloat16(), torch.randn(rows, I, device="cuda").bfloat16()
+    dgu, g = activation.glu_bwd_both_raw(d, gu, act)
+    assert torch.equal(g, activation.glu_fwd_raw(gu, act)) and torch.equal(dgu, activation.glu_bwd_raw(d, gu, act))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("first", [0, 1, 3])
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 4097, 1 << 20])
+def test_squared_norm_of_any_alignment(dtype, first, n):
+    """fp32 sums in some order: 2^-23 for each of the at most n / threads + log steps, here a generous 1e-5."""
+    import ctypes
+    from trainscale_b200.ops import _lib
+    torch.manual_seed(0)
+    x = torch.randn(n + first, device="cuda").to(dtype)[first:]
+    out = torch.zeros(1, device="cuda")
+    rc = _lib.load("elementwise").ts_sumsq(_lib.ptr(x), int(dtype == torch.bfloat16), ctypes.c_longlong(n), _lib.ptr(out), _lib.ptr(None),
+                                           ctypes.c_float(0.5), _lib.stream_ptr())
+    assert rc == 0
+    ref = (x.double() * 0.5).square().sum()
+    assert abs(float(out) - float(ref)) <= 1e-5 * float(ref)

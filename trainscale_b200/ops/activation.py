@@ -40,6 +40,17 @@ def glu_bwd_raw(d, gu, act_id: int):
     return dgu
 
 
+def glu_bwd_both_raw(d, gu, act_id: int):
+    """(gradient of gate|up, the gated product itself) in one pass over gate|up."""
+    lib = _lib.load("elementwise")
+    I = gu.shape[1] // 2
+    dgu, out = torch.empty_like(gu), torch.empty(gu.shape[0], I, dtype=gu.dtype, device=gu.device)
+    rc = lib.ts_glu_bwd_both(_lib.ptr(d), _lib.ptr(gu), _lib.ptr(dgu), _lib.ptr(out), ctypes.c_longlong(gu.shape[0]), I, 2 * I,
+                             act_id, _lib.stream_ptr())
+    _lib.check(rc, "ts_glu_bwd_both")
+    return dgu, out
+
+
 class _GluFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, gate_up, act):

@@ -55,9 +55,13 @@ class _GluLinearFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dout):
         gu, w = ctx.saved_tensors
-        g = activation.glu_fwd_raw(gu, ctx.act_id)                                   # rebuilt, never stored
-        dg, dw = gemm.linear_bwd(dout, g, w, True, ctx.needs_input_grad[1])
-        return activation.glu_bwd_raw(dg.reshape(-1, g.shape[1]), gu, ctx.act_id).view(ctx.in_shape), dw, None
+        dg = gemm.matmul_nn(dout, w)
+        if not ctx.needs_input_grad[1]:
+            return activation.glu_bwd_raw(dg, gu, ctx.act_id).view(ctx.in_shape), None, None
+        # the product is rebuilt, never stored, in the pass that needs gate and up anyway
+        dgu, g = activation.glu_bwd_both_raw(dg, gu, ctx.act_id)
+        _, dw = gemm.linear_bwd(dout, g, w, False, True)
+        return dgu.view(ctx.in_shape), dw, None
 
 
 def supported(x: torch.Tensor, *weights: torch.Tensor) -> bool:
