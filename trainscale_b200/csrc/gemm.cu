@@ -696,8 +696,12 @@ extern "C" int ts_gemm_bf16_act(const void* A, const void* B, void* C, int M, in
     const int tiles256 = ((M + 127) / 128) * ((N + 255) / 256);
     bn = (N >= 256 && tiles256 >= sm_count()) ? 256 : (N >= 128 ? 128 : 64);
     if (N >= 256 && tiles256 < sm_count() && ((M + 127) / 128) * ((N + 127) / 128) < tiles256 * 2) bn = 128;
-    // the paired-CTA kernel wins whenever every CTA pair gets at least one 256 x 256 tile
-    if (N >= 256 && M >= 256 && ((M + 255) / 256) * ((N + 255) / 256) >= sm_count() / 2) bn = 512;
+    // the paired-CTA kernel wins whenever every CTA pair gets at least one 256 x 256 tile, and where 128 x 128 tiles are more than
+    // one for every SM: they take two rounds for what a pair does in one (1000 x 4096 x 4096 35.6 / 29.2 us; one round is the
+    // better one: 500 x 3072 x 2048 13.3 / 17.4)
+    if (N >= 256 && M >= 256 && (((M + 255) / 256) * ((N + 255) / 256) >= sm_count() / 2 ||
+                                 ((M + 127) / 128) * ((N + 127) / 128) > sm_count()))
+      bn = 512;
   }
   const bool two_cta = (bn == 512);
   if (two_cta) bn = 128;   // per-CTA B box: 128 rows of N
