@@ -108,3 +108,35 @@ def test_squared_norm_of_any_alignment(dtype, first, n):
     assert rc == 0
     ref = (x.double() * 0.5).square().sum()
     assert abs(float(out) - float(ref)) <= 1e-5 * float(ref)
+
+
+# places per chunk of 32: one, a whole chunk and its neighbours, runs that cross one or many chunks, that begin or end on a border
+@pytest.mark.parametrize("ids", [[3], [5] * 31 + [6], [1] * 32, [1] * 33, [2] * 16 + [4] * 40 + [7], [0] * 300, list(range(100)),
+                                 [1] * 32 + [2] * 64 + [3] * 5, "random"])
+@pytest.mark.parametrize("H", [8, 1032])
+@pytest.mark.parametrize("added", [False, True])
+def test_embedding_gradient_in_the_owners_rows(ids, H, added):
+    """fp32 sums of bf16 rows: 2^-23 of the magnitudes for each term; rows of no token keep what they had."""
+    from trainscale_b200.ops.embedding import TokenEmbedding
+    torch.manual_seed(0)
+    V = 400
+    flat = torch.randint(0, V, (700,)) if ids == "random" else torch.tensor(ids)
+    flat = flat[torch.randperm(len(flat))].cuda()
+    emb = TokenEmbedding(V, H).to("cuda", torch.bfloat16)
+    w, runs = emb.weight, []
+    w._ts_unit = object()                              # as an engine's parameter has one
+    dy = torch.randn(1, len(flat), H, device="cuda").bfloat16()
+    before = torch.randn(V, H, device="cuda")
+    for _ in range(2):
+        w.main_grad, w.grad_added = before.clone(), added
+        emb(flat.view(1, -1)).backward(dy)
+        assert w.grad is None and w.grad_added
+        runs.append(w.main_grad)
+    assert torch.equal(*runs)
+    base = before.double() if added else torch.zeros(V, H, device="cuda", dtype=torch.double)
+    ref = base.index_add(0, flat, dy[0].double())
+    size = base.abs().index_add(0, flat, dy[0].double().abs())
+    assert ((runs[0].double() - ref).abs() <= 2.0 ** -23 * (len(flat) + 1) * size + 1e-30).all()
+    del w.main_grad
+    emb(flat.view(1, -1)).backward(dy)                 # without an owner: torch's own gradient
+    assert w.grad is not None

@@ -979,6 +979,82 @@ __global__ void sumsq_kernel(const T* __restrict__ x, long long n, float* __rest
   }
 }
 
+// Gradient of an embedding, added to fp32 rows: grad[v] += sum of dy[t] over the tokens t with id v.  `ids` are sorted, `order` the
+// tokens they came from (stable, so sums have one order and the same bits every time).  Instead of a dense bf16 matrix that is
+// zeroed, scattered into, converted and added, only rows that occur are touched.  A CTA takes EMB_CHUNK sorted places and 8 columns
+// per thread; runs of one id that lie inside the chunk are added to their row, the ends of longer ones are left as partial rows
+// (part[2 c]: of the run that comes from the chunk before, part[2 c + 1]: of the one that goes on) for the second kernel.
+constexpr int EMB_CHUNK = 32, EMB_THREADS = 128, EMB_AHEAD = 8;
+__device__ __forceinline__ void add_row8(float* dst, const float (&a)[8]) {
+  float4 x = *reinterpret_cast<float4*>(dst), y = *reinterpret_cast<float4*>(dst + 4);
+  x.x += a[0]; x.y += a[1]; x.z += a[2]; x.w += a[3];
+  y.x += a[4]; y.y += a[5]; y.z += a[6]; y.w += a[7];
+  *reinterpret_cast<float4*>(dst) = x;
+  *reinterpret_cast<float4*>(dst + 4) = y;
+}
+__device__ __forceinline__ void put_row8(float* dst, const float (&a)[8]) {
+  *reinterpret_cast<float4*>(dst) = make_float4(a[0], a[1], a[2], a[3]);
+  *reinterpret_cast<float4*>(dst + 4) = make_float4(a[4], a[5], a[6], a[7]);
+}
+
+__global__ void __launch_bounds__(EMB_THREADS) embedding_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const int* __restrict__ ids,
+                                                                    const long long* __restrict__ order, float* __restrict__ grad,
+                                                                    float* __restrict__ part, int T, int H) {
+  const int col = (blockIdx.y * EMB_THREADS + threadIdx.x) * 8;
+  if (col >= H) return;
+  const int first = blockIdx.x * EMB_CHUNK, end = min(T, first + EMB_CHUNK);
+  const bool from_before = first > 0 && ids[first - 1] == ids[first];
+  float acc[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+  bool head = from_before;                       // the current run began in an earlier chunk
+  for (int i0 = first; i0 < end; i0 += EMB_AHEAD) {
+    bf16x8 raw[EMB_AHEAD];
+#pragma unroll
+    for (int k = 0; k < EMB_AHEAD; ++k)
+      if (i0 + k < end) raw[k] = *reinterpret_cast<const bf16x8*>(dy + order[i0 + k] * H + col);
+#pragma unroll
+    for (int k = 0; k < EMB_AHEAD; ++k) {
+      const int i = i0 + k;
+      if (i >= end) break;
+      float v[8];
+      unpack8(raw[k], v);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[e] += v[e];
+      const int id = ids[i];
+      const bool goes_on = i + 1 < T && ids[i + 1] == id;
+      if (goes_on && i + 1 < end) continue;
+      if (head) put_row8(part + static_cast<size_t>(2 * blockIdx.x) * H + col, acc);
+      else if (goes_on) put_row8(part + static_cast<size_t>(2 * blockIdx.x + 1) * H + col, acc);
+      else add_row8(grad + static_cast<size_t>(id) * H + col, acc);
+      head = false;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+    }
+  }
+}
+
+// one CTA column per chunk whose last run began in it and goes on: its parts, in order
+__global__ void __launch_bounds__(EMB_THREADS) embedding_bwd_join_kernel(const int* __restrict__ ids, const float* __restrict__ part,
+                                                                         float* __restrict__ grad, int T, int H, int chunks) {
+  const int col = (blockIdx.y * EMB_THREADS + threadIdx.x) * 8, c = blockIdx.x, last = (c + 1) * EMB_CHUNK - 1;
+  if (col >= H || last + 1 >= T) return;
+  const int id = ids[last];
+  if (ids[last + 1] != id) return;
+  if (c > 0 && ids[c * EMB_CHUNK] == id && ids[c * EMB_CHUNK - 1] == id) return;      // it began before: that chunk joins it
+  float acc[8];
+  const float* p = part + static_cast<size_t>(2 * c + 1) * H + col;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) acc[e] = p[e];
+  for (int d = c + 1; d < chunks && ids[d * EMB_CHUNK] == id; ++d) {
+    const float4* q = reinterpret_cast<const float4*>(part + static_cast<size_t>(2 * d) * H + col);
+    const float4 x = q[0], y = q[1];
+    acc[0] += x.x; acc[1] += x.y; acc[2] += x.z; acc[3] += x.w;
+    acc[4] += y.x; acc[5] += y.y; acc[6] += y.z; acc[7] += y.w;
+  }
+  add_row8(grad + static_cast<size_t>(id) * H + col, acc);
+}
+
 // dst (+)= src * mul with dtype conversion (gradient accumulate / cast helper)
 template <typename D, typename S>
 __global__ void scale_cast_kernel(D* __restrict__ dst, const S* __restrict__ src, long long n, float mul,
@@ -1246,6 +1322,20 @@ extern "C" int ts_sumsq(const void* x, int is_bf16, long long n, float* out, flo
     sumsq_kernel<bf16><<<grid, 512, 0, ST(stream)>>>((const bf16*)x, n, out, nonfinite_flag, mul);
   else
     sumsq_kernel<float><<<grid, 512, 0, ST(stream)>>>((const float*)x, n, out, nonfinite_flag, mul);
+  return (int)cudaGetLastError();
+}
+
+// grad [V][H] += sums of dy [T][H] by id; part: fp32 workspace of 2 * ceil(T / 32) * H values (ts_embedding_bwd_parts rows).
+extern "C" int ts_embedding_bwd_parts(int T) { return 2 * ((T + EMB_CHUNK - 1) / EMB_CHUNK); }
+extern "C" int ts_embedding_bwd(const void* dy, const int* sorted_ids, const long long* order, float* grad, float* part, int T, int H,
+                                void* stream) {
+  if (T <= 0) return 0;
+  if (H <= 0 || H % 8 || ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(grad) | reinterpret_cast<uintptr_t>(part)) & 15u))
+    return -10;
+  const int chunks = (T + EMB_CHUNK - 1) / EMB_CHUNK;
+  const dim3 grid((unsigned)chunks, (unsigned)((H + EMB_THREADS * 8 - 1) / (EMB_THREADS * 8)));
+  embedding_bwd_kernel<<<grid, EMB_THREADS, 0, ST(stream)>>>((const bf16*)dy, sorted_ids, order, grad, part, T, H);
+  if (chunks > 1) embedding_bwd_join_kernel<<<grid, EMB_THREADS, 0, ST(stream)>>>(sorted_ids, part, grad, T, H, chunks);
   return (int)cudaGetLastError();
 }
 

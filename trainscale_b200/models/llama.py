@@ -21,6 +21,7 @@ import torch.nn.functional as F
 from torch.utils.checkpoint import checkpoint
 
 from ..ops import activation, attention, cross_entropy, fused_blocks, gemm, norm, rope
+from ..ops.embedding import TokenEmbedding
 from ..utils import recompute as _recompute_switch
 
 
@@ -323,7 +324,7 @@ class LlamaModel(nn.Module):
         """`layer_range`: build only these decoder layers (one pipeline stage's); the others are placeholders."""
         super().__init__()
         self.cfg = cfg
-        self.embed_tokens = nn.Embedding(cfg.vocab_size, cfg.hidden_size)
+        self.embed_tokens = TokenEmbedding(cfg.vocab_size, cfg.hidden_size)
         self.layers = nn.ModuleList(LlamaDecoderLayer(cfg) if (layer_range is None or i in layer_range) else nn.Identity()
                                     for i in range(cfg.num_hidden_layers))
         self.norm = RMSNorm(cfg.hidden_size, cfg.rms_norm_eps, cfg.norm_weight_offset)
