@@ -121,7 +121,7 @@ __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint3
 // to DEC_MAX_CLUSTER in distributed shared memory, more through partial results [seq][Hq][split][D] fp32 and lse
 // [seq][Hq][split] for decode_merge_kernel.
 // One warp per key with shuffled dot products / this (32 query heads of 8 kv heads, us; at the copy bandwidth): 64 sequences of
-// 300 keys of 64 75 / 14.5 (6.1), of 2000 keys of 128 571 / 101 (81), 4 of 10000 keys of 128 249 / 37 (25), 1 of 100 of 64 16 / 5.
+// 300 keys of 64 75 / 14.5 (6.1), of 2000 keys of 128 571 / 96 (81), 4 of 10000 keys of 128 249 / 34 (25), 1 of 100 of 64 16 / 5.
 template <int D, bool CLUSTER>
 __global__ void __launch_bounds__(DEC_WARPS * 32)
 decode_attention_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, const __nv_bfloat16* __restrict__ k_cache,
@@ -157,69 +157,83 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, const
     for (int e = 0; e < 4; ++e) acc[n][e] = 0.f;
   const int kv_width = Hkv * D;
   const int* table = block_table + static_cast<size_t>(seq) * max_blocks;
-  // first cache row of a 16-key tile whose keys lie in one block; one past the end repeats the last one, masked below.  The
-  // block table is read two steps ahead and the next step's lines are asked into L2, so that a step waits for L2 only
+  // first cache row of a 16-key tile whose keys lie in one block; one past the end repeats the last one, masked below.  A step's
+  // keys are loaded as soon as the products with the keys before have read their registers, its values likewise; the lines come
+  // from L2, into which they are asked a step earlier, and the block table is read three steps ahead
   const bool whole = (block_size & 15) == 0;
   constexpr int STRIDE = DEC_WARPS * 16 * KT;
   auto tile_base = [&](int t) { return min(t, (t1 - 1) & ~15); };
   auto tile_first = [&](int t) {
     const int base = tile_base(t);
-    return whole ? table[base / block_size] * static_cast<long long>(block_size) + base % block_size : 0ll;
+    return whole ? table[base / block_size] * block_size + base % block_size : 0;
   };
-  long long cur[KT], next[KT], later[KT];
-  if (t0 + warp * 16 * KT < t1) {
+  auto row_at = [&](int base, int first, int j) {
+    const int key = min(base + j, t1 - 1);
+    const int slot = whole ? first + (key - base) : table[key / block_size] * block_size + key % block_size;
+    return static_cast<size_t>(slot) * kv_width + hk * D;
+  };
+  uint4 kr[KT][2][NK], vr[KT][4][NV];
+  auto load_k = [&](int t, const int (&first)[KT]) {
 #pragma unroll
-    for (int x = 0; x < KT; ++x) {
-      cur[x] = tile_first(t0 + (warp * KT + x) * 16);
-      next[x] = tile_first(t0 + (warp * KT + x) * 16 + STRIDE);
-    }
-  }
-  for (int t = t0 + warp * 16 * KT; t < t1; t += STRIDE) {
-#pragma unroll
-    for (int x = 0; x < KT; ++x) later[x] = tile_first(t + 2 * STRIDE + x * 16);
-    uint4 kr[KT][2][NK], vr[KT][4][NV];
-#pragma unroll
-    for (int x = 0; x < KT; ++x) {
-      const int base = tile_base(t + x * 16);
-      auto row = [&](int j) {
-        const int key = min(base + j, t1 - 1);
-        const size_t slot = whole ? cur[x] + (key - base) : static_cast<size_t>(table[key / block_size]) * block_size + key % block_size;
-        return slot * kv_width + hk * D;
-      };
+    for (int x = 0; x < KT; ++x)
 #pragma unroll
       for (int n = 0; n < 2; ++n) {
-        const __nv_bfloat16* p = k_cache + row(n * 8 + gid) + tig * 8;
+        const __nv_bfloat16* p = k_cache + row_at(tile_base(t + x * 16), first[x], n * 8 + gid) + tig * 8;
 #pragma unroll
         for (int i = 0; i < NK; ++i) kr[x][n][i] = *reinterpret_cast<const uint4*>(p + i * 32);
       }
+  };
+  auto load_v = [&](int t, const int (&first)[KT]) {
+#pragma unroll
+    for (int x = 0; x < KT; ++x)
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const __nv_bfloat16* p = v_cache + row((j >> 1) * 8 + tig * 2 + (j & 1)) + gid * 8;
+        const __nv_bfloat16* p = v_cache + row_at(tile_base(t + x * 16), first[x], (j >> 1) * 8 + tig * 2 + (j & 1)) + gid * 8;
 #pragma unroll
         for (int i = 0; i < NV; ++i) vr[x][j][i] = *reinterpret_cast<const uint4*>(p + i * 64);
       }
+  };
+  const int begin = t0 + warp * 16 * KT;
+  int next[KT], later[KT];
+  if (begin < t1) {
+    int first[KT];
+#pragma unroll
+    for (int x = 0; x < KT; ++x) {
+      first[x] = tile_first(begin + x * 16);
+      next[x] = tile_first(begin + STRIDE + x * 16);
+      later[x] = tile_first(begin + 2 * STRIDE + x * 16);
     }
+    load_k(begin, first);
+    load_v(begin, first);
+  }
+  for (int t = begin; t < t1; t += STRIDE) {
+    int far[KT];
+#pragma unroll
+    for (int x = 0; x < KT; ++x) far[x] = tile_first(t + 3 * STRIDE + x * 16);
     if (whole) {
       // 32 lines of keys and of values: rows of one 128-byte line each (D = 64, two tiles) or of two (D = 128)
       const int x = KT == 2 ? lane >> 4 : 0, j = KT == 2 ? lane & 15 : lane >> 1;
-      const int key = min(tile_base(t + STRIDE + x * 16) + j, t1 - 1);
-      const size_t at = (next[x] + (key - tile_base(t + STRIDE + x * 16))) * kv_width + hk * D + (KT == 2 ? 0 : (lane & 1) * 64);
+      const size_t at = row_at(tile_base(t + 2 * STRIDE + x * 16), KT == 2 && x ? later[KT - 1] : later[0], j) + (KT == 2 ? 0 : (lane & 1) * 64);
       asm volatile("prefetch.global.L2 [%0];" ::"l"(k_cache + at));
       asm volatile("prefetch.global.L2 [%0];" ::"l"(v_cache + at));
     }
+    float sc[KT][2][4];
 #pragma unroll
-    for (int x = 0; x < KT; ++x) {
-      float s[2][4];
+    for (int x = 0; x < KT; ++x)
 #pragma unroll
       for (int n = 0; n < 2; ++n) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) s[n][e] = 0.f;
+        for (int e = 0; e < 4; ++e) sc[x][n][e] = 0.f;
 #pragma unroll
         for (int i = 0; i < NK; ++i) {
-          mma_bf16_16816(s[n], qv[i].x, 0u, qv[i].y, 0u, kr[x][n][i].x, kr[x][n][i].y);
-          mma_bf16_16816(s[n], qv[i].z, 0u, qv[i].w, 0u, kr[x][n][i].z, kr[x][n][i].w);
+          mma_bf16_16816(sc[x][n], qv[i].x, 0u, qv[i].y, 0u, kr[x][n][i].x, kr[x][n][i].y);
+          mma_bf16_16816(sc[x][n], qv[i].z, 0u, qv[i].w, 0u, kr[x][n][i].z, kr[x][n][i].w);
         }
       }
+    if (t + STRIDE < t1) load_k(t + STRIDE, next);
+#pragma unroll
+    for (int x = 0; x < KT; ++x) {
+      float (&s)[2][4] = sc[x];
       const int k0 = t + x * 16 + tig * 2;
       float mn = m;
 #pragma unroll
@@ -265,10 +279,11 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, const
         }
       }
     }
+    if (t + STRIDE < t1) load_v(t + STRIDE, next);
 #pragma unroll
     for (int x = 0; x < KT; ++x) {
-      cur[x] = next[x];
       next[x] = later[x];
+      later[x] = far[x];
     }
   }
   l += __shfl_xor_sync(0xffffffffu, l, 1);
@@ -405,8 +420,8 @@ static int launch_decode(const void* q, int q_stride, const void* k_cache, const
 
 // Shares of a sequence's keys: 256 CTAs in all, at least 128 keys each.  Up to eight are merged inside the kernel; more (long
 // sequences, few heads) cost a second launch and are taken where the eight would have more than 512 keys each.  Measured (us by
-// splits, 8 kv heads): 1 x 10000 keys of 128 27 (8) / 16 (32), 4 x 10000 59 (4) / 37 (8) / 43 (16), 64 x 300 keys of 64
-// 14.5 (1) / 20 (2), 1 x 1000 13 (1) / 6 (8).
+// splits, 8 kv heads): 1 x 10000 keys of 128 28 (8) / 18 (32), 4 x 10000 55 (4) / 34 (8) / 41 (16), 64 x 300 keys of 64
+// 12.5 (1) / 20 (2), 1 x 1000 11 (1) / 6 (8).
 extern "C" int ts_decode_splits(int num_seqs, int Hkv, int max_len) {
   const long long ctas = static_cast<long long>(num_seqs) * Hkv;
   int want = ctas > 0 ? static_cast<int>((256 + ctas - 1) / ctas) : 1;
