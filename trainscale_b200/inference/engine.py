@@ -439,7 +439,8 @@ class ModelRunner:
         c = self.cfg
         return (self.use_graphs and self.lora is None and host.all_single and len(host.q_lens) <= 256
                 and host.out_rows == list(range(len(host.q_lens)))
-                and (self.own_layers or (c.head_dim in (64, 128) and getattr(c, "num_local_experts", 0) == 0)))
+                and (self.own_layers or (c.head_dim in (64, 128) and self.Hq // self.Hkv <= MAX_DECODE_GROUP
+                                         and getattr(c, "num_local_experts", 0) == 0)))
 
     # index tensors of a captured step: name -> (dtype, value of a padding row)
     def _static_fields(self) -> dict:

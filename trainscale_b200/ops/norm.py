@@ -105,7 +105,8 @@ STEP_ROWS = 1024     # rows up to which a CTA per row (ts_rmsnorm_step) is taken
 
 @torch.no_grad()
 def rmsnorm_step(x: torch.Tensor, w: torch.Tensor, eps: float, residual: torch.Tensor | None = None, w_offset: float = 0.0):
-    """`rmsnorm` of the rows of a serving step, without autograd."""
+    """`rmsnorm` of the rows of a serving step, without autograd.  `w` may be fetched while the kernels before this one still run,
+    back to the last ordinary launch: none of these may be what writes it."""
     H = x.shape[-1]
     if not (x.is_cuda and x.dtype == w.dtype == torch.bfloat16 and H % 8 == 0 and H <= 8192 and x.dim() == 2
             and 0 < x.shape[0] <= STEP_ROWS and (residual is None or residual.shape == x.shape and residual.dtype == x.dtype)
