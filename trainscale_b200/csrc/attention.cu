@@ -1045,6 +1045,8 @@ extern "C" int ts_flash_fwd(const void* q, const void* k, const void* v, void* o
 // Portions of prompts against keys of a cache: sequence b's queries are rows [cu_q[b], cu_q[b + 1]) of q and the LAST of its
 // k_lens[b] keys, which lie at rows k_starts[b] on of k / v (head g of k at column g * D, of v too); rows up to the next
 // multiple of 128 are read, so they hold finite values.  Causal.  Weights keep 16 bits (SPLIT).
+// Tensor-bound (the split is half as much again as plain bf16 weights): 0.65 ms for 8192 query rows of up to 10000 keys, 32 / 8 heads of
+// 128; three such prompts with 24 decoding steps took 438 ms with fp32 scores in memory, 101 ms with this.
 extern "C" int ts_flash_portions(const void* q, const void* k, const void* v, void* o, long long q_rows, long long k_rows,
                                  int q_stride, int kv_stride, int o_stride, int Hq, int Hkv, int D, int B, const int* cu_q,
                                  const int* k_starts, const int* k_lens, int max_q, float scale, void* stream) {
