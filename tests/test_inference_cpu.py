@@ -222,3 +222,40 @@ def test_tensor_parallel_serving_matches_single_process():
     r = subprocess.run(cmd, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
     assert "RESULT inference tp=2" in r.stdout and "ok=True" in r.stdout
+
+
+def _core(max_len, **cfg):
+    from dataclasses import replace
+    from trainscale_b200.inference.engine import EngineCore
+    model = build_model(replace(CFG, **cfg), dtype=torch.float32, seed=1)
+    return EngineCore(EngineConfig(model="tiny", device="cpu", dtype="float32",
+                                   cache=CacheConfig(block_size=16, num_gpu_blocks=64, max_model_len=max_len)), model=model), model
+
+
+def test_positions_beyond_the_rotary_tables_are_refused():
+    """Kernels read cos and sin by position: a sequence may not outgrow the tables, and the refusal leaves the cache as it was."""
+    import pytest
+    from trainscale_b200.inference.batch import HostBatch, StepEntry
+    core, _ = _core(32, max_position_embeddings=64)
+    assert core.runner.cos.shape[0] == 64
+    core.execute([StepEntry(0, [5] * 60)])
+    free = core.cache.alloc.num_free
+    for tokens in ([7] * 5, [7] * 100):
+        with pytest.raises(ValueError, match="longer than the 64 positions"):
+            core.execute([StepEntry(0, tokens), StepEntry(1, [3])])
+    assert core.cache.alloc.num_free == free and core.cache.seqs[0].num_tokens == 60 and 1 not in core.cache.seqs
+    core.execute([StepEntry(0, [7] * 4)])
+    # the runner's own entry points refuse a batch that was made past the engine
+    with pytest.raises(ValueError, match="longer than the 64 positions"):
+        core.runner.forward(HostBatch(core.cache, [StepEntry(0, [7])]).to_device("cpu"))
+
+
+def test_rotary_tables_cover_the_longest_sequence_of_the_engine():
+    from trainscale_b200.inference.batch import StepEntry
+    core, model = _core(200, max_position_embeddings=64)
+    assert core.runner.cos.shape[0] >= 200
+    ids = torch.randint(0, CFG.vocab_size, (150,), generator=torch.Generator().manual_seed(2)).tolist()
+    core.execute([StepEntry(0, ids[:100], [])])
+    got = core.execute([StepEntry(0, ids[100:])])
+    want = model(torch.tensor([ids])).logits[0, -1]
+    assert torch.allclose(got[0], want, atol=1e-4, rtol=1e-4)

@@ -278,3 +278,26 @@ def test_chained_steps_wait_for_their_rows():
     want = run(False)
     for _ in range(5):
         assert torch.equal(run(True), want)
+
+
+def test_sequences_cross_the_default_rotary_tables():
+    """A model that declares 8192 positions, served to 8300: prompt portions and decoding rows on both sides of the border."""
+    from trainscale_b200.inference import engine as E
+    from trainscale_b200.inference.batch import StepEntry
+    from trainscale_b200.models.llama import LlamaConfig, build_model
+    cfg = LlamaConfig(vocab_size=300, hidden_size=128, intermediate_size=256, num_hidden_layers=1, num_attention_heads=2,
+                      num_key_value_heads=1, head_dim=64)
+    model = build_model(cfg, dtype=torch.bfloat16, device="cuda", seed=1)
+    core = E.EngineCore(E.EngineConfig(model="tiny", cache=E.CacheConfig(block_size=16, num_gpu_blocks=600, max_model_len=8300)),
+                        model=model)
+    assert cfg.max_position_embeddings == 8192 and core.runner.cos.shape[0] >= 8300
+    ids = torch.randint(0, 300, (8300,), generator=torch.Generator().manual_seed(3)).tolist()
+    want = model(torch.tensor([ids], device="cuda")).logits[0].float().detach()
+    at = 0
+    for n in (8100, 90, 1, 1, 1, 1, 104, 1, 1):
+        row = core.execute([StepEntry(0, ids[at:at + n])])[0]
+        at += n
+        assert (row - want[at - 1]).norm() <= 0.02 * want[at - 1].norm(), at
+    assert at == 8300
+    with pytest.raises(ValueError):
+        core.execute([StepEntry(0, [1] * (core.runner.cos.shape[0] - at + 1))])

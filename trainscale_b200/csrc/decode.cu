@@ -381,7 +381,8 @@ extern "C" int ts_kv_cache_write(const void* qkv, int row_stride, int k_col0, in
   return (int)cudaGetLastError();
 }
 
-// D a multiple of 16; rows of qkv (q | k | v heads) 16-byte aligned; cos / sin: fp32 [positions][D / 2]; slot < 0: not cached.
+// D a multiple of 16; rows of qkv (q | k | v heads) 16-byte aligned; cos / sin: fp32 [positions][D / 2], read at pos[row] without
+// a check: the caller refuses sequences longer than the tables (inference/engine.py check_length); slot < 0: not cached.
 extern "C" int ts_rope_cache(void* qkv, long long row_stride, const float* cos_t, const float* sin_t, const int* pos,
                              const long long* slot_mapping, void* k_cache, void* v_cache, long long rows, int Hq, int Hkv, int D,
                              void* stream) {

@@ -262,10 +262,11 @@ class ModelRunner:
     """Runs a decoder over a flattened token batch with the paged cache.  A model that defines `serve(batch, cache)` brings
     its own layers (models/mezilix.py); for `LlamaForCausalLM` they are here."""
 
-    def __init__(self, model, cache: PagedKVCache, device, tp=None, use_graphs: bool = False):
+    def __init__(self, model, cache: PagedKVCache, device, tp=None, use_graphs: bool = False, max_len: int = 0):
         """`tp`: tensor-parallel context of a model sharded with `shard_model_for_tensor_parallel` (every rank runs
         the same batch; the attention and MLP outputs are all-reduced).  `use_graphs`: pure decode steps replay a CUDA
-        graph per (padded batch size, block-table width) instead of launching ~12 kernels per layer from Python."""
+        graph per (padded batch size, block-table width) instead of launching ~12 kernels per layer from Python.
+        `max_len`: longest sequence that has to be served, where it is more than the rotary tables hold by default."""
         self.model, self.cache, self.device = model.eval(), cache, torch.device(device)
         self.cfg = model.config
         self.own_layers = hasattr(model, "serve")
@@ -275,12 +276,18 @@ class ModelRunner:
             self.use_graphs = bool(use_graphs) and self.device.type == "cuda"
         else:
             self.cuda = self.device.type == "cuda" and next(model.parameters()).dtype == torch.bfloat16
-            self.cos, self.sin = model.model.rope_tables(self.device, min(self.cfg.max_position_embeddings, 1 << 16))
+            self.cos, self.sin = model.model.rope_tables(self.device, max(min(self.cfg.max_position_embeddings, 1 << 16), max_len))
             ws = self.tp.size if self.tp is not None else 1
             self.Hq, self.Hkv = self.cfg.num_attention_heads // ws, self.cfg.num_key_value_heads // ws
             self.use_graphs = bool(use_graphs) and self.cuda
         self.graphs: dict = {}
         self.graph_replays = 0
+
+    def check_length(self, longest: int) -> None:
+        """Refuses sequences of more tokens than the rotary tables have rows: the kernels read cos and sin by position, unchecked."""
+        if not self.own_layers and longest > self.cos.shape[0]:
+            raise ValueError(f"a sequence of {longest} tokens is longer than the {self.cos.shape[0]} positions this engine was "
+                             "built for (cache.max_model_len)")
 
     def _reduce(self, x: torch.Tensor) -> torch.Tensor:
         if self.tp is not None:
@@ -431,6 +438,7 @@ class ModelRunner:
     @torch.no_grad()
     def forward(self, batch: StepBatch) -> torch.Tensor:
         """Hidden state of every wanted row [wanted, H]."""
+        self.check_length(batch.max_len)
         return self._layers(batch)
 
     # ---------------------------------------------------------------- CUDA-graph decode
@@ -459,6 +467,7 @@ class ModelRunner:
         while n_pad < n:
             n_pad *= 2
         bt, sl = self.cache.block_table(host.seq_ids, None)
+        self.check_length(int(sl.max()))
         width = -(-bt.shape[1] // 32) * 32
         key = (n_pad, width)
         st = self.graphs.get(key)
@@ -610,7 +619,8 @@ class EngineCore:
         self.cache = PagedKVCache(c.num_hidden_layers, nb, cc.block_size, dtype=dtype, device=self.device,
                                   enable_prefix_caching=cc.enable_prefix_caching, spec=spec,
                                   state_slots=config.scheduler.max_num_seqs)
-        self.runner = ModelRunner(self.model, self.cache, self.device, tp=self.tp, use_graphs=not config.enforce_eager)
+        self.runner = ModelRunner(self.model, self.cache, self.device, tp=self.tp, use_graphs=not config.enforce_eager,
+                                  max_len=cc.max_model_len)
         self.waiting: deque[_Request] = deque()
         self.running: list[_Request] = []
         self.metrics = MetricsAggregator()
@@ -693,6 +703,8 @@ class EngineCore:
             if not e.tokens or any(not 0 <= w < len(e.tokens) for w in e.wanted):
                 raise ValueError("an entry needs tokens, and the wanted places lie among them")
             self._check_tokens(e.tokens)
+            held = self.cache.seqs.get(e.seq_id)
+            self.runner.check_length((held.num_tokens if held else 0) + len(e.tokens))
         if len({e.seq_id for e in entries}) != len(entries):
             raise ValueError("a sequence may appear once in a step")
         need = sum(self.cache.blocks_needed(e.seq_id, len(e.tokens)) for e in entries)
