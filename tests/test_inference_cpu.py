@@ -259,3 +259,20 @@ def test_rotary_tables_cover_the_longest_sequence_of_the_engine():
     got = core.execute([StepEntry(0, ids[100:])])
     want = model(torch.tensor([ids])).logits[0, -1]
     assert torch.allclose(got[0], want, atol=1e-4, rtol=1e-4)
+
+
+def test_windows_and_capped_scores_are_served_as_the_model_computes_them():
+    """Prompts, portions and decoding rows on both sides of the window's border against the whole-sequence forward."""
+    from trainscale_b200.inference.batch import StepEntry
+    for cfg in (dict(sliding_window=24), dict(attn_logit_softcap=0.5), dict(sliding_window=17, attn_logit_softcap=0.5)):
+        core, model = _core(128, initializer_range=0.2, **cfg)
+        plain = _core(128, initializer_range=0.2)[0]
+        ids = torch.randint(0, CFG.vocab_size, (60,), generator=torch.Generator().manual_seed(2)).tolist()
+        want = model(torch.tensor([ids])).logits[0]
+        at = 0
+        for n in (20, 1, 3, 1, 30, 1, 1, 3):
+            got = core.execute([StepEntry(0, ids[at:at + n])])[0]
+            other = plain.execute([StepEntry(0, ids[at:at + n])])[0]
+            at += n
+            assert torch.allclose(got, want[at - 1], atol=1e-3, rtol=1e-3), (cfg, at)
+        assert not torch.allclose(other, want[at - 1], atol=1e-2, rtol=1e-2), cfg         # the mask or cap does count here

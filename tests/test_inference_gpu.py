@@ -301,3 +301,68 @@ def test_sequences_cross_the_default_rotary_tables():
     assert at == 8300
     with pytest.raises(ValueError):
         core.execute([StepEntry(0, [1] * (core.runner.cos.shape[0] - at + 1))])
+
+
+# windows: smaller than a 16-key tile, no multiple of one, of a tile and of a 128-key block; never reached; a cap with and without
+@pytest.mark.parametrize("window,softcap", [(5, 0.0), (100, 0.0), (128, 3.0), (500, 0.0), (None, 3.0)])
+@pytest.mark.parametrize("graphs", [False, True])
+def test_windows_and_capped_scores_on_every_path(window, softcap, graphs):
+    """First prompts, portions, decoding rows of their own and beside portions, launched and captured, against the whole-sequence
+    forward of the same kernels' training path (bf16 rounding of two layers: 2e-2 of the norm, as above)."""
+    from trainscale_b200.inference import engine as E
+    from trainscale_b200.inference.batch import StepEntry
+    from trainscale_b200.models.llama import LlamaConfig, build_model
+    cfg = LlamaConfig(vocab_size=300, hidden_size=256, intermediate_size=512, num_hidden_layers=2, num_attention_heads=4,
+                      num_key_value_heads=2, head_dim=64, sliding_window=window, attn_logit_softcap=softcap, initializer_range=0.1)
+    model = build_model(cfg, dtype=torch.bfloat16, device="cuda", seed=1)
+    core = E.EngineCore(E.EngineConfig(model="tiny", enforce_eager=not graphs,
+                                       cache=E.CacheConfig(block_size=16, num_gpu_blocks=256, max_model_len=1024)), model=model)
+    g = torch.Generator().manual_seed(3)
+    ids = {s: torch.randint(0, 300, (n,), generator=g).tolist() for s, n in ((0, 450), (1, 150))}
+    want = {s: model(torch.tensor([t], device="cuda")).logits[0].float().detach() for s, t in ids.items()}
+    at = {s: 0 for s in ids}
+    for step in ([(0, 210), (1, 90)], [(0, 1), (1, 1)], [(0, 130), (1, 1)], [(0, 1), (1, 40)], [(0, 1), (1, 1)], [(0, 99), (1, 7)],
+                 [(0, 1), (1, 1)]):
+        logits = core.execute([StepEntry(s, ids[s][at[s]:at[s] + n]) for s, n in step])
+        for (s, n), row in zip(step, logits):
+            at[s] += n
+            ref = want[s][at[s] - 1]
+            assert (row - ref).norm() <= 0.02 * ref.norm(), (s, at[s])
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("lens,splits,window,softcap", [([1, 16, 17, 700], 1, 16, 0.0), ([5, 130, 127, 900], 3, 100, 2.0),
+                                                        ([2000, 63, 65, 64], 8, 1001, 0.0), ([2000, 1500, 20, 64], 12, 1500, 0.0),
+                                                        ([300, 20, 1, 64], 2, 0, 1.5)])
+def test_decode_attention_of_a_window_matches_fp64(D, lens, splits, window, softcap):
+    """Bounds as without a window; keys before it hold NaN in rows that share no tile with visible ones."""
+    import ctypes
+    from trainscale_b200.ops import _lib
+    torch.manual_seed(2)
+    dev, bs, Hq, Hkv, n = "cuda", 16, 6, 2, len(lens)
+    kw = Hkv * D
+    blocks = [-(-k // bs) for k in lens]
+    kc, vc = (torch.randn(sum(blocks) + 1, bs, Hkv, D, device=dev, dtype=torch.bfloat16) for _ in range(2))
+    table = torch.full((n, max(blocks)), sum(blocks), dtype=torch.int32)
+    for i, part in enumerate(torch.randperm(sum(blocks)).split(blocks)):
+        table[i, :blocks[i]] = part
+        first = max(0, lens[i] - window) // bs if window else 0
+        kc[part[:first]] = vc[part[:first]] = float("nan")
+    table = table.to(dev)
+    q = torch.randn(n, Hq * D + 2 * kw, device=dev, dtype=torch.bfloat16)
+    out = torch.empty(n, Hq * D, device=dev, dtype=torch.bfloat16)
+    po, pl = torch.empty(n, Hq, splits, D, device=dev), torch.empty(n, Hq, splits, device=dev)
+    rc = _lib.load("decode").ts_decode_attention_ex(
+        _lib.ptr(q), q.stride(0), _lib.ptr(kc), _lib.ptr(vc), _lib.ptr(table), table.shape[1],
+        _lib.ptr(torch.tensor(lens, dtype=torch.int32, device=dev)), _lib.ptr(out), Hq * D, _lib.ptr(po), _lib.ptr(pl), n, Hq, Hkv, D,
+        bs, 16, splits, ctypes.c_float(1 / math.sqrt(D)), window, ctypes.c_float(softcap), _lib.stream_ptr())
+    assert rc == 0
+    for i, m in enumerate(lens):
+        lo = max(0, m - window) if window else 0
+        k, v = (c[table[i, :blocks[i]].long()].reshape(-1, Hkv, D)[lo:m].double().repeat_interleave(Hq // Hkv, 1) for c in (kc, vc))
+        sc = torch.einsum("hd,khd->hk", q[i, :Hq * D].double().view(Hq, D), k) / math.sqrt(D)
+        if softcap:
+            sc = softcap * torch.tanh(sc / softcap)
+        ref = torch.einsum("hk,khd->hd", torch.softmax(sc, -1), v).reshape(-1)
+        err = (out[i].double() - ref).abs()
+        assert (err <= 2.0 ** -8 * ref.abs() + 2.0 ** -15 * 5).all(), (i, float(err.max()))

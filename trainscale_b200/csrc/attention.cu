@@ -1044,12 +1044,13 @@ extern "C" int ts_flash_fwd(const void* q, const void* k, const void* v, void* o
 
 // Portions of prompts against keys of a cache: sequence b's queries are rows [cu_q[b], cu_q[b + 1]) of q and the LAST of its
 // k_lens[b] keys, which lie at rows k_starts[b] on of k / v (head g of k at column g * D, of v too); rows up to the next
-// multiple of 128 are read, so they hold finite values.  Causal.  Weights keep 16 bits (SPLIT).
+// multiple of 128 are read, so they hold finite values.  Causal; window and softcap as above.  Weights keep 16 bits (SPLIT).
 // Tensor-bound (the split is half as much again as plain bf16 weights): 0.65 ms for 8192 query rows of up to 10000 keys, 32 / 8 heads of
 // 128; three such prompts with 24 decoding steps took 438 ms with fp32 scores in memory, 101 ms with this.
 extern "C" int ts_flash_portions(const void* q, const void* k, const void* v, void* o, long long q_rows, long long k_rows,
                                  int q_stride, int kv_stride, int o_stride, int Hq, int Hkv, int D, int B, const int* cu_q,
-                                 const int* k_starts, const int* k_lens, int max_q, float scale, void* stream) {
+                                 const int* k_starts, const int* k_lens, int max_q, float scale, int window, float softcap,
+                                 void* stream) {
   if ((D != 64 && D != 128) || Hkv <= 0 || Hq % Hkv != 0 || q_rows <= 0 || k_rows <= 0 || B <= 0 || max_q <= 0) return -10;
   CUtensorMap tq, tk, tv;
   int rc = make_tmap_2d(&tq, q, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)q_rows, (uint64_t)Hq * D, (uint64_t)q_stride, 128, 64);
@@ -1061,8 +1062,13 @@ extern "C" int ts_flash_portions(const void* q, const void* k, const void* v, vo
   AttnParams p{};
   p.Hq = Hq; p.Hkv = Hkv; p.group = Hq / Hkv; p.B = B; p.cu_seqlens = cu_q; p.k_starts = k_starts; p.k_lens = k_lens;
   p.causal = 1; p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
+  p.window = window > 0 ? window : 0;
+  p.cap_inv = softcap > 0.f ? scale / softcap : 0.f;
+  p.cap_log2 = softcap > 0.f ? softcap * 1.4426950408889634f : 0.f;
   p.o = (__nv_bfloat16*)o; p.o_stride = o_stride; p.total_rows = q_rows;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (p.window > 0 || p.cap_log2 > 0.f)
+    return D == 128 ? launch_fwd<128, true, true>(tq, tk, tv, p, max_q, st) : launch_fwd<64, true, true>(tq, tk, tv, p, max_q, st);
   return D == 128 ? launch_fwd<128, false, true>(tq, tk, tv, p, max_q, st) : launch_fwd<64, false, true>(tq, tk, tv, p, max_q, st);
 }
 

@@ -122,13 +122,14 @@ __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint3
 // [seq][Hq][split] for decode_merge_kernel.
 // One warp per key with shuffled dot products / this (32 query heads of 8 kv heads, us; at the copy bandwidth): 64 sequences of
 // 300 keys of 64 75 / 14.5 (6.1), of 2000 keys of 128 571 / 96 (81), 4 of 10000 keys of 128 249 / 34 (25), 1 of 100 of 64 16 / 5.
-template <int D, bool CLUSTER>
+// EXT: a window (the last `window` keys, 0: all) or a soft cap of the scores (cap_log2 * tanh(s * cap_inv), cap_log2 0: none).
+template <int D, bool CLUSTER, bool EXT>
 __global__ void __launch_bounds__(DEC_WARPS * 32)
 decode_attention_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, const __nv_bfloat16* __restrict__ k_cache,
                         const __nv_bfloat16* __restrict__ v_cache, const int* __restrict__ block_table,
                         int max_blocks, const int* __restrict__ seq_lens, __nv_bfloat16* __restrict__ out, int out_stride,
                         float* __restrict__ part_out, float* __restrict__ part_lse, int Hq, int Hkv, int block_size,
-                        int chunk, int splits, float scale_log2) {
+                        int chunk, int splits, float scale_log2, int window, float cap_inv, float cap_log2) {
   constexpr int KT = D == 64 ? 2 : 1;      // 16-key tiles in flight: 8 KB of keys and values per warp
   constexpr int NK = D / 32, NV = D / 64;
   const int split = blockIdx.x, hk = blockIdx.y, seq = blockIdx.z;
@@ -137,8 +138,9 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, const
   grid_trigger();
   grid_wait();
   const int len = seq_lens[seq];
-  const int share = (max(chunk, (len + splits - 1) / splits) + 15) & ~15;
-  const int t0 = split * share, t1 = min(len, t0 + share);
+  const int seen = EXT && window > 0 ? max(0, len - window) : 0, base0 = seen & ~15;      // first visible key, and its tile
+  const int share = (max(chunk, (len - base0 + splits - 1) / splits) + 15) & ~15;
+  const int t0 = base0 + split * share, t1 = min(len, t0 + share);
   __shared__ __align__(16) float s_acc[DEC_WARPS][DEC_MAX_GROUP][D];
   __shared__ float s_m[DEC_WARPS][DEC_MAX_GROUP], s_l[DEC_WARPS][DEC_MAX_GROUP];
   __shared__ __align__(16) float c_acc[DEC_MAX_GROUP][D];      // the CTA's result, not normalised
@@ -240,7 +242,8 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, const
       for (int n = 0; n < 2; ++n)
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          s[n][e] = k0 + n * 8 + e < t1 ? s[n][e] * scale_log2 : -INFINITY;
+          s[n][e] = EXT && cap_log2 > 0.f ? cap_log2 * tanhf(s[n][e] * cap_inv) : s[n][e] * scale_log2;
+          if (k0 + n * 8 + e >= t1 || (EXT && k0 + n * 8 + e < seen)) s[n][e] = -INFINITY;
           mn = fmaxf(mn, s[n][e]);
         }
       mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 1));
@@ -407,14 +410,15 @@ extern "C" int ts_kv_gather(const void* k_cache, const void* v_cache, const int*
 
 namespace ts {
 
-template <int D, bool CLUSTER>
+template <int D, bool CLUSTER, bool EXT>
 static int launch_decode(const void* q, int q_stride, const void* k_cache, const void* v_cache, const int* block_table,
                          int max_blocks, const int* seq_lens, void* out, int out_stride, float* part_out, float* part_lse,
-                         int num_seqs, int Hq, int Hkv, int block_size, int chunk, int splits, float scale_log2, cudaStream_t st) {
-  return launch_chained(decode_attention_kernel<D, CLUSTER>, dim3(splits, Hkv, num_seqs), dim3(DEC_WARPS * 32), 0, st,
+                         int num_seqs, int Hq, int Hkv, int block_size, int chunk, int splits, float scale_log2, int window,
+                         float cap_inv, float cap_log2, cudaStream_t st) {
+  return launch_chained(decode_attention_kernel<D, CLUSTER, EXT>, dim3(splits, Hkv, num_seqs), dim3(DEC_WARPS * 32), 0, st,
                         CLUSTER ? splits : 1, true, (const __nv_bfloat16*)q, q_stride, (const __nv_bfloat16*)k_cache,
                         (const __nv_bfloat16*)v_cache, block_table, max_blocks, seq_lens, (__nv_bfloat16*)out, out_stride, part_out,
-                        part_lse, Hq, Hkv, block_size, chunk, splits, scale_log2);
+                        part_lse, Hq, Hkv, block_size, chunk, splits, scale_log2, window, cap_inv, cap_log2);
 }
 
 }  // namespace ts
@@ -434,27 +438,41 @@ extern "C" int ts_decode_splits(int num_seqs, int Hkv, int max_len) {
 
 // chunk: least number of keys of a split (multiples of 16 keep whole cache blocks together); splits * chunk may exceed the keys.
 // splits > 8 (DEC_MAX_CLUSTER): part_out fp32 [num_seqs][Hq][splits][D], part_lse fp32 [num_seqs][Hq][splits] (caller-provided
-// workspace); else they are not used.
-extern "C" int ts_decode_attention(const void* q, int q_stride, const void* k_cache, const void* v_cache,
-                                   const int* block_table, int max_blocks, const int* seq_lens, void* out,
-                                   int out_stride, float* part_out, float* part_lse, int num_seqs, int Hq, int Hkv,
-                                   int D, int block_size, int chunk, int splits, float scale, void* stream) {
+// workspace); else they are not used.  window > 0: the last `window` keys of a sequence only; softcap > 0: scaled scores become
+// softcap * tanh(score / softcap).
+extern "C" int ts_decode_attention_ex(const void* q, int q_stride, const void* k_cache, const void* v_cache,
+                                      const int* block_table, int max_blocks, const int* seq_lens, void* out,
+                                      int out_stride, float* part_out, float* part_lse, int num_seqs, int Hq, int Hkv,
+                                      int D, int block_size, int chunk, int splits, float scale, int window, float softcap,
+                                      void* stream) {
   if (num_seqs <= 0) return 0;
   if (Hkv <= 0 || Hq % Hkv != 0 || Hq / Hkv > DEC_MAX_GROUP || (D != 64 && D != 128) || splits <= 0 || num_seqs > 65535 ||
       Hkv > 65535)
     return -10;
   if (q_stride % 8 || (reinterpret_cast<uintptr_t>(q) & 15u)) return -11;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  const float sl = scale * 1.4426950408889634f;
+  const float log2e = 1.4426950408889634f;
   const bool cluster = splits <= DEC_MAX_CLUSTER;
-  auto launch = D == 128 ? (cluster ? launch_decode<128, true> : launch_decode<128, false>)
-                         : (cluster ? launch_decode<64, true> : launch_decode<64, false>);
+  auto launch = D == 128 ? (cluster ? launch_decode<128, true, false> : launch_decode<128, false, false>)
+                         : (cluster ? launch_decode<64, true, false> : launch_decode<64, false, false>);
+  if (window > 0 || softcap > 0.f)
+    launch = D == 128 ? (cluster ? launch_decode<128, true, true> : launch_decode<128, false, true>)
+                      : (cluster ? launch_decode<64, true, true> : launch_decode<64, false, true>);
   const int rc = launch(q, q_stride, k_cache, v_cache, block_table, max_blocks, seq_lens, out, out_stride, part_out, part_lse,
-                        num_seqs, Hq, Hkv, block_size, chunk, splits, sl, st);
+                        num_seqs, Hq, Hkv, block_size, chunk, splits, scale * log2e, window, softcap > 0.f ? scale / softcap : 0.f,
+                        softcap > 0.f ? softcap * log2e : 0.f, st);
   if (rc || cluster) return rc;
   if (D == 128)
     decode_merge_kernel<128><<<dim3(num_seqs, Hq), 128, 0, st>>>(part_out, part_lse, (__nv_bfloat16*)out, out_stride, Hq, splits);
   else
     decode_merge_kernel<64><<<dim3(num_seqs, Hq), 64, 0, st>>>(part_out, part_lse, (__nv_bfloat16*)out, out_stride, Hq, splits);
   return (int)cudaGetLastError();
+}
+
+extern "C" int ts_decode_attention(const void* q, int q_stride, const void* k_cache, const void* v_cache,
+                                   const int* block_table, int max_blocks, const int* seq_lens, void* out,
+                                   int out_stride, float* part_out, float* part_lse, int num_seqs, int Hq, int Hkv,
+                                   int D, int block_size, int chunk, int splits, float scale, void* stream) {
+  return ts_decode_attention_ex(q, q_stride, k_cache, v_cache, block_table, max_blocks, seq_lens, out, out_stride, part_out, part_lse,
+                                num_seqs, Hq, Hkv, D, block_size, chunk, splits, scale, 0, 0.f, stream);
 }

@@ -352,44 +352,50 @@ class ModelRunner:
         Hq, Hkv, D = self.Hq, self.Hkv, c.head_dim
         scale = 1.0 / math.sqrt(D)
         T = qkv2d.shape[0]
+        # as the model's own forward; a window that no sequence of the step outgrows hides nothing
+        window = c.sliding_window if c.sliding_window and batch.max_len > c.sliding_window else 0
+        seen = (window, float(c.attn_logit_softcap or 0.0))
         if self.cuda and fresh and D in (64, 128):
             # every sequence starts at position 0: packed-prompt flash attention
-            o, _ = flash.flash_forward_only(qkv2d.unsqueeze(0), Hq, Hkv, D, True, scale, batch.cu_q, max(q_lens))
+            o, _ = flash.flash_forward_only(qkv2d.unsqueeze(0), Hq, Hkv, D, True, scale, batch.cu_q, max(q_lens), *seen)
             return o.view(T, Hq * D)
         if self.cuda and D in (64, 128) and Hq // Hkv <= MAX_DECODE_GROUP:
             # rows of single tokens come first; the portions of prompts behind them see keys of earlier steps
             out = torch.empty(T, Hq * D, dtype=qkv2d.dtype, device=self.device)
             if batch.n_single:
-                self._attend_rows(layer, qkv2d, batch, out, scale)
+                self._attend_rows(layer, qkv2d, batch, out, scale, *seen)
             if batch.n_single < len(q_lens):
-                self._attend_portions(layer, qkv2d, batch, out, scale)
+                self._attend_portions(layer, qkv2d, batch, out, scale, *seen)
             return out
         # general path (CPU, other head sizes): per sequence against the gathered cache
         outs, off = [], 0
         for sid, n in zip(batch.seq_ids, q_lens):
             q = qkv2d[off:off + n, :Hq * D].view(1, n, Hq, D)
             k, v = self._gathered_kv(layer, sid)
-            o = attention.attention_reference(q, k.unsqueeze(0), v.unsqueeze(0), True, scale)
+            o = attention.attention_reference(q, k.unsqueeze(0), v.unsqueeze(0), True, scale, *seen)
             outs.append(o.reshape(n, Hq * D))
             off += n
         return torch.cat(outs)
 
-    def _attend_rows(self, layer: int, qkv2d: torch.Tensor, batch: StepBatch, out: torch.Tensor, scale: float) -> None:
+    def _attend_rows(self, layer: int, qkv2d: torch.Tensor, batch: StepBatch, out: torch.Tensor, scale: float, window: int,
+                     softcap: float) -> None:
         """out[:n] of the batch's first n rows, single tokens of as many sequences."""
         n, D, table = batch.n_single, self.cfg.head_dim, batch.block_table
         lib = _lib.load("decode")
-        splits = lib.ts_decode_splits(n, self.Hkv, batch.longest_single)
+        longest = batch.longest_single
+        splits = lib.ts_decode_splits(n, self.Hkv, min(longest, window) if window else longest)
         po = pl = None
         if splits > DECODE_CLUSTER:
             po = torch.empty(n, self.Hq, splits, D, dtype=torch.float32, device=self.device)
             pl = torch.empty(n, self.Hq, splits, dtype=torch.float32, device=self.device)
-        rc = lib.ts_decode_attention(
+        rc = lib.ts_decode_attention_ex(
             _lib.ptr(qkv2d), qkv2d.stride(0), _lib.ptr(self.cache.k[layer]), _lib.ptr(self.cache.v[layer]), _lib.ptr(table),
             table.shape[1], _lib.ptr(batch.seq_lens), _lib.ptr(out), out.stride(0), _lib.ptr(po), _lib.ptr(pl), n, self.Hq,
-            self.Hkv, D, self.cache.block_size, 16, splits, ctypes.c_float(scale), _lib.stream_ptr())
-        _lib.check(rc, "ts_decode_attention")
+            self.Hkv, D, self.cache.block_size, 16, splits, ctypes.c_float(scale), window, ctypes.c_float(softcap), _lib.stream_ptr())
+        _lib.check(rc, "ts_decode_attention_ex")
 
-    def _attend_portions(self, layer: int, qkv2d: torch.Tensor, batch: StepBatch, out: torch.Tensor, scale: float) -> None:
+    def _attend_portions(self, layer: int, qkv2d: torch.Tensor, batch: StepBatch, out: torch.Tensor, scale: float, window: int,
+                         softcap: float) -> None:
         """out of the rows behind the single tokens: portions of prompts that continue what earlier steps left in the cache.
         Their sequences' keys and values are laid side by side in key order, as many sequences at a time as
         GATHER_ROWS allows, and go through the flash kernel."""
@@ -402,7 +408,8 @@ class ModelRunner:
                 _lib.ptr(self.cache.k[layer]), _lib.ptr(self.cache.v[layer]), _lib.ptr(table), table.shape[1],
                 _lib.ptr(g.starts), _lib.ptr(lens), g.end - g.first, g.longest, bs, kw, _lib.ptr(kv), _lib.stream_ptr())
             _lib.check(rc, "ts_kv_gather")
-            flash.flash_portions(qkv2d, kv[:, :kw], kv[:, kw:], out, self.Hq, self.Hkv, D, g.cu_q, g.starts, lens, g.max_q, scale)
+            flash.flash_portions(qkv2d, kv[:, :kw], kv[:, kw:], out, self.Hq, self.Hkv, D, g.cu_q, g.starts, lens, g.max_q, scale,
+                                 window, softcap)
 
     def _layers(self, batch: StepBatch) -> torch.Tensor:
         """The decoder over a flattened token batch; returns the final-norm hidden state of the wanted rows."""

@@ -91,22 +91,24 @@ def flash_attention_qkv(qkv: torch.Tensor, n_heads: int, n_kv_heads: int, head_d
 
 
 def flash_forward_only(qkv: torch.Tensor, n_heads: int, n_kv_heads: int, head_dim: int, causal: bool = True,
-                       scale: float | None = None, cu_seqlens: torch.Tensor | None = None, max_seqlen: int | None = None):
+                       scale: float | None = None, cu_seqlens: torch.Tensor | None = None, max_seqlen: int | None = None,
+                       window: int = 0, softcap: float = 0.0):
     """(out [B,S,Hq*D], lse [Hq, B*S]) without autograd."""
     B, S, W = qkv.shape
     scale = scale if scale is not None else 1.0 / math.sqrt(head_dim)
     q2 = qkv.reshape(B * S, W)
     if cu_seqlens is not None:
         cu = cu_seqlens.to(torch.int32)
-        o, lse = _fwd(q2, n_heads, n_kv_heads, head_dim, cu.numel() - 1, 0, cu, int(max_seqlen or B * S), causal, scale)
+        o, lse = _fwd(q2, n_heads, n_kv_heads, head_dim, cu.numel() - 1, 0, cu, int(max_seqlen or B * S), causal, scale,
+                      window, softcap)
     else:
-        o, lse = _fwd(q2, n_heads, n_kv_heads, head_dim, B, S, None, S, causal, scale)
+        o, lse = _fwd(q2, n_heads, n_kv_heads, head_dim, B, S, None, S, causal, scale, window, softcap)
     return o.view(B, S, -1), lse
 
 
 def flash_portions(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tensor, n_heads: int, n_kv_heads: int,
                    head_dim: int, cu_q: torch.Tensor, k_starts: torch.Tensor, k_lens: torch.Tensor, max_q: int,
-                   scale: float) -> None:
+                   scale: float, window: int = 0, softcap: float = 0.0) -> None:
     """Causal attention of portions of sequences against all of their keys, without autograd: queries q[cu_q[b]:cu_q[b + 1],
     :Hq * D] are the last of the k_lens[b] keys at rows k_starts[b] on of k and v [rows, Hkv * D] (same row stride; rows up to
     the next multiple of 128 hold finite values); results go to the same rows of `out`.  Offsets and lengths are int32."""
@@ -115,5 +117,5 @@ def flash_portions(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch
     rc = _lib.load("attention").ts_flash_portions(
         _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(out), _ll(q.shape[0]), _ll(k.shape[0]), q.stride(0), k.stride(0),
         out.stride(0), n_heads, n_kv_heads, head_dim, k_starts.numel(), _lib.ptr(cu_q), _lib.ptr(k_starts), _lib.ptr(k_lens),
-        max_q, _f(scale), _lib.stream_ptr())
+        max_q, _f(scale), int(window), _f(float(softcap)), _lib.stream_ptr())
     _lib.check(rc, "ts_flash_portions")
