@@ -109,21 +109,27 @@ __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint3
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// the leading eight bits of a value, and those of two as an operand word
+__device__ __forceinline__ float high_part(float x) { return __uint_as_float(__float_as_uint(x) & 0xffff0000u); }
+__device__ __forceinline__ uint32_t pack_high(float x, float y) { return __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632); }
+__device__ __forceinline__ void put_float4(float* dst, const float* v) { *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]); }
+
 // grid (splits, Hkv, sequences).  A CTA takes an even share of one sequence's keys for one kv head and all query heads that share
 // it.  Memory should bound this; scalar code for four heads of 128 spends 5 - 10 times as many issue slots per key as the loads
 // leave (shuffles of the dot products, conversions), so both products are warp MMAs whose operands come straight from global
 // memory as 16-byte vectors:
 //   S = Q K^T  rows are heads; a lane's eight consecutive dimensions feed two reduction steps (Q in the same order)
 //   O += P V   a lane has the same dimensions of four keys, two keys of one dimension are one operand word; P comes from S in
-//              registers.  The heads use eight of the sixteen rows, so the rows 8 - 15 hold what the bf16 weights of rows 0 - 7
-//              leave over: weights keep 16 bits at no cost
+//              registers, cut into three bf16 parts of eight bits each, which hold all of an fp32 weight.  The heads use eight
+//              of the sixteen rows, so rows 8 - 15 take the second part; up to four heads are given twice (rows 4 - 7 repeat
+//              rows 0 - 3) and rows 4 - 7 take the third, more (WIDE) need a second product for it
 // Every warp walks its own 16-key tiles with a softmax state of its own; states meet in shared memory, then over the splits: up
 // to DEC_MAX_CLUSTER in distributed shared memory, more through partial results [seq][Hq][split][D] fp32 and lse
 // [seq][Hq][split] for decode_merge_kernel.
 // One warp per key with shuffled dot products / this (32 query heads of 8 kv heads, us; at the copy bandwidth): 64 sequences of
 // 300 keys of 64 75 / 14.5 (6.1), of 2000 keys of 128 571 / 96 (81), 4 of 10000 keys of 128 249 / 34 (25), 1 of 100 of 64 16 / 5.
 // EXT: a window (the last `window` keys, 0: all) or a soft cap of the scores (cap_log2 * tanh(s * cap_inv), cap_log2 0: none).
-template <int D, bool CLUSTER, bool EXT>
+template <int D, bool CLUSTER, bool EXT, bool WIDE>
 __global__ void __launch_bounds__(DEC_WARPS * 32)
 decode_attention_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, const __nv_bfloat16* __restrict__ k_cache,
                         const __nv_bfloat16* __restrict__ v_cache, const int* __restrict__ block_table,
@@ -135,6 +141,8 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, const
   const int split = blockIdx.x, hk = blockIdx.y, seq = blockIdx.z;
   const int group = Hq / Hkv;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
+  const int head = WIDE ? gid : gid & 3;           // of this lane's row
+  const bool third = !WIDE && gid >= 4;            // whose weights are the third parts
   grid_trigger();
   grid_wait();
   const int len = seq_lens[seq];
@@ -149,9 +157,9 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, const
   uint4 qv[NK];
 #pragma unroll
   for (int i = 0; i < NK; ++i)
-    qv[i] = gid < group ? *reinterpret_cast<const uint4*>(q + static_cast<size_t>(seq) * q_stride + (hk * group + gid) * D + i * 32 + tig * 8)
-                        : make_uint4(0u, 0u, 0u, 0u);
-  float m = -INFINITY, l = 0.f;            // of head gid; l of this lane's keys
+    qv[i] = head < group ? *reinterpret_cast<const uint4*>(q + static_cast<size_t>(seq) * q_stride + (hk * group + head) * D + i * 32 + tig * 8)
+                         : make_uint4(0u, 0u, 0u, 0u);
+  float m = -INFINITY, l = 0.f;            // of the lane's head; l of this lane's keys
   float acc[NV * 8][4];                    // [n]: columns 2 tig, 2 tig + 1 <-> dimensions 64 (n / 8) + 8 column + n % 8
 #pragma unroll
   for (int n = 0; n < NV * 8; ++n)
@@ -258,14 +266,19 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, const
           for (int e = 0; e < 4; ++e) acc[n][e] *= a;
         m = mn;
       }
-      uint32_t high[2], low[2];
+      uint32_t a0[2], a8[2], last[2];        // operand words of rows gid and gid + 8; the third parts
 #pragma unroll
       for (int n = 0; n < 2; ++n) {
         const float p0 = fast_ex2(s[n][0] - sub), p1 = fast_ex2(s[n][1] - sub);
         l += p0 + p1;
-        high[n] = pack_bf16x2(p0, p1);
-        const float2 h = unpack_bf16x2(high[n]);
-        low[n] = pack_bf16x2(p0 - h.x, p1 - h.y);
+        const float r0 = p0 - high_part(p0), r1 = p1 - high_part(p1);
+        a0[n] = pack_high(p0, p1);
+        a8[n] = pack_high(r0, r1);
+        last[n] = pack_bf16x2(r0 - high_part(r0), r1 - high_part(r1));
+        if (third) {
+          a0[n] = last[n];
+          a8[n] = 0u;
+        }
       }
 #pragma unroll
       for (int i = 0; i < NV; ++i) {
@@ -275,10 +288,14 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, const
                                   {vr[x][3][i].x, vr[x][3][i].y, vr[x][3][i].z, vr[x][3][i].w}};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          mma_bf16_16816(acc[i * 8 + 2 * e], high[0], low[0], high[1], low[1], __byte_perm(v[0][e], v[1][e], 0x5410),
-                         __byte_perm(v[2][e], v[3][e], 0x5410));
-          mma_bf16_16816(acc[i * 8 + 2 * e + 1], high[0], low[0], high[1], low[1], __byte_perm(v[0][e], v[1][e], 0x7632),
-                         __byte_perm(v[2][e], v[3][e], 0x7632));
+          const uint32_t b0[2] = {__byte_perm(v[0][e], v[1][e], 0x5410), __byte_perm(v[2][e], v[3][e], 0x5410)};
+          const uint32_t b1[2] = {__byte_perm(v[0][e], v[1][e], 0x7632), __byte_perm(v[2][e], v[3][e], 0x7632)};
+          mma_bf16_16816(acc[i * 8 + 2 * e], a0[0], a8[0], a0[1], a8[1], b0[0], b0[1]);
+          mma_bf16_16816(acc[i * 8 + 2 * e + 1], a0[0], a8[0], a0[1], a8[1], b1[0], b1[1]);
+          if (WIDE) {
+            mma_bf16_16816(acc[i * 8 + 2 * e], last[0], 0u, last[1], 0u, b0[0], b0[1]);
+            mma_bf16_16816(acc[i * 8 + 2 * e + 1], last[0], 0u, last[1], 0u, b1[0], b1[1]);
+          }
         }
       }
     }
@@ -291,20 +308,24 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, const
   }
   l += __shfl_xor_sync(0xffffffffu, l, 1);
   l += __shfl_xor_sync(0xffffffffu, l, 2);
-  if (tig == 0) {
-    s_m[warp][gid] = m;
-    s_l[warp][gid] = l;
+  if (tig == 0 && !third) {
+    s_m[warp][head] = m;
+    s_l[warp][head] = l;
   }
 #pragma unroll
   for (int i = 0; i < NV; ++i)
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
-      float* dst = &s_acc[warp][gid][i * 64 + (2 * tig + c) * 8];
+      float sum[8];
 #pragma unroll
-      for (int n = 0; n < 8; n += 4)
-        *reinterpret_cast<float4*>(dst + n) =
-            make_float4(acc[i * 8 + n][c] + acc[i * 8 + n][c + 2], acc[i * 8 + n + 1][c] + acc[i * 8 + n + 1][c + 2],
-                        acc[i * 8 + n + 2][c] + acc[i * 8 + n + 2][c + 2], acc[i * 8 + n + 3][c] + acc[i * 8 + n + 3][c + 2]);
+      for (int n = 0; n < 8; ++n) {
+        const float x = acc[i * 8 + n][c];
+        sum[n] = (WIDE ? 0.f : __shfl_down_sync(0xffffffffu, x, 16)) + acc[i * 8 + n][c + 2] + x;     // smallest parts first
+      }
+      if (third) continue;
+      float* dst = &s_acc[warp][head][i * 64 + (2 * tig + c) * 8];
+      put_float4(dst, sum);
+      put_float4(dst + 4, sum + 4);
     }
   __syncthreads();
   for (int idx = threadIdx.x; idx < group * D; idx += blockDim.x) {
@@ -410,15 +431,21 @@ extern "C" int ts_kv_gather(const void* k_cache, const void* v_cache, const int*
 
 namespace ts {
 
-template <int D, bool CLUSTER, bool EXT>
+template <int D, bool CLUSTER, bool EXT, bool WIDE>
 static int launch_decode(const void* q, int q_stride, const void* k_cache, const void* v_cache, const int* block_table,
                          int max_blocks, const int* seq_lens, void* out, int out_stride, float* part_out, float* part_lse,
                          int num_seqs, int Hq, int Hkv, int block_size, int chunk, int splits, float scale_log2, int window,
                          float cap_inv, float cap_log2, cudaStream_t st) {
-  return launch_chained(decode_attention_kernel<D, CLUSTER, EXT>, dim3(splits, Hkv, num_seqs), dim3(DEC_WARPS * 32), 0, st,
+  return launch_chained(decode_attention_kernel<D, CLUSTER, EXT, WIDE>, dim3(splits, Hkv, num_seqs), dim3(DEC_WARPS * 32), 0, st,
                         CLUSTER ? splits : 1, true, (const __nv_bfloat16*)q, q_stride, (const __nv_bfloat16*)k_cache,
                         (const __nv_bfloat16*)v_cache, block_table, max_blocks, seq_lens, (__nv_bfloat16*)out, out_stride, part_out,
                         part_lse, Hq, Hkv, block_size, chunk, splits, scale_log2, window, cap_inv, cap_log2);
+}
+
+template <int D, bool CLUSTER>
+static auto pick_decode(bool ext, bool wide) {
+  return ext ? (wide ? launch_decode<D, CLUSTER, true, true> : launch_decode<D, CLUSTER, true, false>)
+             : (wide ? launch_decode<D, CLUSTER, false, true> : launch_decode<D, CLUSTER, false, false>);
 }
 
 }  // namespace ts
@@ -453,11 +480,9 @@ extern "C" int ts_decode_attention_ex(const void* q, int q_stride, const void* k
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const float log2e = 1.4426950408889634f;
   const bool cluster = splits <= DEC_MAX_CLUSTER;
-  auto launch = D == 128 ? (cluster ? launch_decode<128, true, false> : launch_decode<128, false, false>)
-                         : (cluster ? launch_decode<64, true, false> : launch_decode<64, false, false>);
-  if (window > 0 || softcap > 0.f)
-    launch = D == 128 ? (cluster ? launch_decode<128, true, true> : launch_decode<128, false, true>)
-                      : (cluster ? launch_decode<64, true, true> : launch_decode<64, false, true>);
+  const bool ext = window > 0 || softcap > 0.f, wide = Hq / Hkv > 4;
+  auto launch = D == 128 ? (cluster ? pick_decode<128, true>(ext, wide) : pick_decode<128, false>(ext, wide))
+                         : (cluster ? pick_decode<64, true>(ext, wide) : pick_decode<64, false>(ext, wide));
   const int rc = launch(q, q_stride, k_cache, v_cache, block_table, max_blocks, seq_lens, out, out_stride, part_out, part_lse,
                         num_seqs, Hq, Hkv, block_size, chunk, splits, scale * log2e, window, softcap > 0.f ? scale / softcap : 0.f,
                         softcap > 0.f ? softcap * log2e : 0.f, st);
