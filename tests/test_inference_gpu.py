@@ -405,3 +405,48 @@ def test_decode_weights_keep_fp32(Hq, Hkv, D, splits):
     exact = -left / (3 + torch.exp(s.double()))                     # (the values' own rest)
     err = (out.view(n, Hkv, Hq // Hkv, D).double() - exact.view(n, Hkv, 1, 1)).abs()
     assert float(err.max()) <= 3 * 2.0 ** -22 / 3, float(err.max())
+
+
+@pytest.mark.parametrize("Hq,Hkv,D", [(4, 1, 64), (16, 2, 128), (3, 3, 64)])
+@pytest.mark.parametrize("window", [0, 40])
+@pytest.mark.parametrize("splits", [1, 3, 12])
+def test_decode_attention_keeps_infinite_values(Hq, Hkv, D, window, splits):
+    """An infinite value that is seen, with a weight that any number of bits may hold, makes its dimension infinite and no other;
+    one that is not seen (before the window, in the same tile) none.  The largest weight is one, whose lower parts are zero."""
+    import ctypes
+    from trainscale_b200.ops import _lib
+    torch.manual_seed(4)
+    dev, bs, lens = "cuda", 16, [1, 16, 17, 47, 300]
+    n, blocks = len(lens), [-(-k // bs) for k in lens]
+    kc, vc = (torch.randn(sum(blocks), bs, Hkv, D, device=dev, dtype=torch.bfloat16) for _ in range(2))
+    table = torch.zeros(n, max(blocks), dtype=torch.int32)
+    for i, part in enumerate(torch.randperm(sum(blocks)).split(blocks)):
+        table[i, :blocks[i]] = part
+    table = table.to(dev)
+
+    def put(i, key, d, value):
+        vc[table[i, key // bs], key % bs, :, d] = value
+
+    for i, m in enumerate(lens):
+        put(i, m - 1, 3, math.inf)                                        # the last key
+        put(i, max(0, m - 20), 5, -math.inf)
+        put(i, max(0, m - 12), 6, math.nan)
+        if window and m > window and (m - window) % bs:
+            put(i, m - window - 1, 7, math.inf)
+    q = torch.randn(n, Hq * D, device=dev, dtype=torch.bfloat16)
+    out = torch.empty_like(q)
+    po, pl = torch.empty(n, Hq, splits, D, device=dev), torch.empty(n, Hq, splits, device=dev)
+    rc = _lib.load("decode").ts_decode_attention_ex(
+        _lib.ptr(q), Hq * D, _lib.ptr(kc), _lib.ptr(vc), _lib.ptr(table), table.shape[1],
+        _lib.ptr(torch.tensor(lens, dtype=torch.int32, device=dev)), _lib.ptr(out), Hq * D, _lib.ptr(po), _lib.ptr(pl), n, Hq, Hkv, D,
+        bs, 16, splits, ctypes.c_float(1 / math.sqrt(D)), window, ctypes.c_float(0), _lib.stream_ptr())
+    assert rc == 0
+    for i, m in enumerate(lens):
+        lo = max(0, m - window) if window else 0
+        k, v = (c[table[i, :blocks[i]].long()].reshape(-1, Hkv, D)[lo:m].double().repeat_interleave(Hq // Hkv, 1) for c in (kc, vc))
+        w = torch.softmax(torch.einsum("hd,khd->hk", q[i].double().view(Hq, D), k) / math.sqrt(D), -1)
+        ref = (w.t().unsqueeze(-1) * v).sum(0).reshape(-1)
+        got = out[i].double()
+        assert torch.equal(got.isinf() * got.sign(), ref.isinf() * ref.sign()) and torch.equal(got.isnan(), ref.isnan()), (i, m)
+        fine = ref.isfinite()
+        assert ((got - ref).abs()[fine] <= 2.0 ** -8 * ref.abs()[fine] + 2.0 ** -20 * 5).all(), (i, m)

@@ -111,6 +111,8 @@ __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint3
 
 // the leading eight bits of a value, and those of two as an operand word
 __device__ __forceinline__ float high_part(float x) { return __uint_as_float(__float_as_uint(x) & 0xffff0000u); }
+// and what they leave, at least `least`
+__device__ __forceinline__ float rest_part(float x, float least) { return fmaxf(x - high_part(x), least); }
 __device__ __forceinline__ uint32_t pack_high(float x, float y) { return __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632); }
 __device__ __forceinline__ void put_float4(float* dst, const float* v) { *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]); }
 
@@ -120,7 +122,8 @@ __device__ __forceinline__ void put_float4(float* dst, const float* v) { *reinte
 // memory as 16-byte vectors:
 //   S = Q K^T  rows are heads; a lane's eight consecutive dimensions feed two reduction steps (Q in the same order)
 //   O += P V   a lane has the same dimensions of four keys, two keys of one dimension are one operand word; P comes from S in
-//              registers, cut into three bf16 parts of eight bits each, which hold all of an fp32 weight.  The heads use eight
+//              registers, cut into three bf16 parts of eight bits each, which hold all of an fp32 weight.  No part of a weight is
+//              zero (2^-24 of it at least): an infinite value stays infinite in every product.  The heads use eight
 //              of the sixteen rows, so rows 8 - 15 take the second part; up to four heads are given twice (rows 4 - 7 repeat
 //              rows 0 - 3) and rows 4 - 7 take the third, more (WIDE) need a second product for it
 // Every warp walks its own 16-key tiles with a softmax state of its own; states meet in shared memory, then over the splits: up
@@ -202,6 +205,18 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, const
 #pragma unroll
         for (int i = 0; i < NV; ++i) vr[x][j][i] = *reinterpret_cast<const uint4*>(p + i * 64);
       }
+    if (t + KT * 16 > t1 || (EXT && t < seen)) {
+      // keys that do not count: their weights are zero, their values must be too (an infinite one would give NaN)
+#pragma unroll
+      for (int x = 0; x < KT; ++x)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int key = t + x * 16 + (j >> 1) * 8 + tig * 2 + (j & 1);
+          if (key >= t1 || (EXT && key < seen))
+#pragma unroll
+            for (int i = 0; i < NV; ++i) vr[x][j][i] = make_uint4(0u, 0u, 0u, 0u);
+        }
+    }
   };
   const int begin = t0 + warp * 16 * KT;
   int next[KT], later[KT];
@@ -271,10 +286,11 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, const
       for (int n = 0; n < 2; ++n) {
         const float p0 = fast_ex2(s[n][0] - sub), p1 = fast_ex2(s[n][1] - sub);
         l += p0 + p1;
-        const float r0 = p0 - high_part(p0), r1 = p1 - high_part(p1);
+        const float r0 = rest_part(p0, p0 * 0x1p-24f), r1 = rest_part(p1, p1 * 0x1p-24f);
         a0[n] = pack_high(p0, p1);
         a8[n] = pack_high(r0, r1);
-        last[n] = pack_bf16x2(r0 - high_part(r0), r1 - high_part(r1));
+        const float x0 = rest_part(r0, p0 * 0x1p-40f), x1 = rest_part(r1, p1 * 0x1p-40f);
+        last[n] = WIDE ? pack_bf16x2(0.5f * x0, 0.5f * x1) : pack_bf16x2(x0, x1);     // (WIDE: in two rows, so that none is zero)
         if (third) {
           a0[n] = last[n];
           a8[n] = 0u;
@@ -293,8 +309,8 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, const
           mma_bf16_16816(acc[i * 8 + 2 * e], a0[0], a8[0], a0[1], a8[1], b0[0], b0[1]);
           mma_bf16_16816(acc[i * 8 + 2 * e + 1], a0[0], a8[0], a0[1], a8[1], b1[0], b1[1]);
           if (WIDE) {
-            mma_bf16_16816(acc[i * 8 + 2 * e], last[0], 0u, last[1], 0u, b0[0], b0[1]);
-            mma_bf16_16816(acc[i * 8 + 2 * e + 1], last[0], 0u, last[1], 0u, b1[0], b1[1]);
+            mma_bf16_16816(acc[i * 8 + 2 * e], last[0], last[0], last[1], last[1], b0[0], b0[1]);
+            mma_bf16_16816(acc[i * 8 + 2 * e + 1], last[0], last[0], last[1], last[1], b1[0], b1[1]);
           }
         }
       }
