@@ -276,3 +276,20 @@ def test_windows_and_capped_scores_are_served_as_the_model_computes_them():
             at += n
             assert torch.allclose(got, want[at - 1], atol=1e-3, rtol=1e-3), (cfg, at)
         assert not torch.allclose(other, want[at - 1], atol=1e-2, rtol=1e-2), cfg         # the mask or cap does count here
+
+
+def test_decode_splits_leave_no_long_share():
+    """However many sequences there are, a long one among them is not left to a CTA per head; shares are not tiny either."""
+    import shutil
+    import pytest
+    from trainscale_b200.ops import _lib
+    if not _lib.lib_path("decode").exists() and shutil.which("nvcc") is None:
+        pytest.skip("needs the built library or nvcc")
+    splits = _lib.load("decode").ts_decode_splits
+    for n in (1, 3, 17, 32, 64, 256, 5000):
+        for heads in (1, 2, 8, 32):
+            for longest in (1, 15, 128, 300, 2000, 9000, 12288, 12289, 60000, 131072):
+                s = splits(n, heads, longest)
+                assert s >= 1 and -(-longest // s) <= 12288 and (s == 1 or longest // s >= 128), (n, heads, longest, s)
+                if longest <= 12288:
+                    assert s <= max(1, -(-256 // (n * heads)))         # even batches fill the GPU once

@@ -100,6 +100,7 @@ kv_gather_kernel(const __nv_bfloat16* __restrict__ k_cache, const __nv_bfloat16*
 constexpr int DEC_WARPS = 4;
 constexpr int DEC_MAX_GROUP = 8;
 constexpr int DEC_MAX_CLUSTER = 8;
+constexpr int DEC_MOST_KEYS = 12288;
 
 __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                                uint32_t b1) {
@@ -466,17 +467,21 @@ static auto pick_decode(bool ext, bool wide) {
 
 }  // namespace ts
 
-// Shares of a sequence's keys: 256 CTAs in all, at least 128 keys each.  Up to eight are merged inside the kernel; more (long
-// sequences, few heads) cost a second launch and are taken where the eight would have more than 512 keys each.  Measured (us by
-// splits, 8 kv heads): 1 x 10000 keys of 128 28 (8) / 18 (32), 4 x 10000 55 (4) / 34 (8) / 41 (16), 64 x 300 keys of 64
-// 12.5 (1) / 20 (2), 1 x 1000 11 (1) / 6 (8).
+// Shares of a sequence's keys: 256 CTAs in all, at least 128 keys each.  Up to eight are merged inside the kernel; more (long sequences, few heads) cost a second
+// launch and are taken where the eight would have more than 512 keys each.  Measured (us by splits, 8 kv heads, nothing cached):
+// 1 x 10000 keys of 128 34 (8) / 28 (32), 4 x 10000 56 (4) / 50 (8) / 56 (16), 64 x 300 keys of 64 25.5 (1) / 31.7 (2), 16 x 300 of
+// 128 17.4 (1, 2) / 24.6 (3).
+// The rule knows the number of sequences and the longest, not the others: one long sequence among many short ones would be left to
+// one CTA per head, 18 us for every 1000 keys of 128.  So no share is longer than DEC_MOST_KEYS: 63 of 100 keys and one of 60000
+// 1018 -> 293 us (5 splits).  Shorter shares cost even batches: 32 x 9000 204 us whole, 218 in two, 222 in three.
 extern "C" int ts_decode_splits(int num_seqs, int Hkv, int max_len) {
   const long long ctas = static_cast<long long>(num_seqs) * Hkv;
   int want = ctas > 0 ? static_cast<int>((256 + ctas - 1) / ctas) : 1;
   const int most = max_len / 128;
   if (want > most) want = most;
   if (want > DEC_MAX_CLUSTER && max_len <= DEC_MAX_CLUSTER * 512) want = DEC_MAX_CLUSTER;
-  return want < 1 ? 1 : want;
+  const int least = static_cast<int>((max_len + static_cast<long long>(DEC_MOST_KEYS) - 1) / DEC_MOST_KEYS);
+  return want > least ? want : least < 1 ? 1 : least;
 }
 
 // chunk: least number of keys of a split (multiples of 16 keep whole cache blocks together); splits * chunk may exceed the keys.
