@@ -450,3 +450,44 @@ def test_decode_attention_keeps_infinite_values(Hq, Hkv, D, window, splits):
         assert torch.equal(got.isinf() * got.sign(), ref.isinf() * ref.sign()) and torch.equal(got.isnan(), ref.isnan()), (i, m)
         fine = ref.isfinite()
         assert ((got - ref).abs()[fine] <= 2.0 ** -8 * ref.abs()[fine] + 2.0 ** -20 * 5).all(), (i, m)
+
+
+def _decode(q, q_stride, kc, vc, table, lens, out, Hq, Hkv, D, bs, splits):
+    import ctypes
+    from trainscale_b200.ops import _lib
+    n = len(lens)
+    po, pl = torch.empty(n, Hq, splits, D, device="cuda"), torch.empty(n, Hq, splits, device="cuda")
+    return _lib.load("decode").ts_decode_attention(
+        _lib.ptr(q), q_stride, _lib.ptr(kc), _lib.ptr(vc), _lib.ptr(table), table.shape[1], _lib.ptr(lens), _lib.ptr(out), Hq * D,
+        _lib.ptr(po), _lib.ptr(pl), n, Hq, Hkv, D, bs, 16, splits, ctypes.c_float(1 / math.sqrt(D)), _lib.stream_ptr())
+
+
+@pytest.mark.parametrize("first,more", [(1, 0), (0, 1), (3, 5), (4, 4)])
+@pytest.mark.parametrize("D", [64, 128])
+def test_decode_attention_of_unaligned_query_rows(first, more, D):
+    """Rows that are no 16-byte vectors give the bits of aligned ones."""
+    torch.manual_seed(0)
+    Hq, Hkv, bs, n = 4, 2, 16, 3
+    kc, vc = (torch.randn(8, bs, Hkv, D, device="cuda").bfloat16() for _ in range(2))
+    table = torch.arange(6, dtype=torch.int32, device="cuda").view(3, 2)
+    lens = torch.tensor([5, 32, 17], dtype=torch.int32, device="cuda")
+    q = torch.randn(n, Hq * D, device="cuda").bfloat16()
+    want, got = torch.empty_like(q), torch.empty_like(q)
+    assert _decode(q, Hq * D, kc, vc, table, lens, want, Hq, Hkv, D, bs, 1) == 0
+    wide = torch.zeros(first + n * (Hq * D + more), device="cuda").bfloat16()
+    rows = wide[first:].view(n, Hq * D + more)[:, :Hq * D]
+    rows.copy_(q)
+    assert _decode(rows, Hq * D + more, kc, vc, table, lens, got, Hq, Hkv, D, bs, 1) == 0
+    assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("splits", [1, 9])
+def test_decode_attention_of_more_sequences_than_a_grid_has(splits):
+    torch.manual_seed(0)
+    n, Hq, D = 65537, 1, 64
+    kc, vc = (torch.randn(3, 16, 1, D, device="cuda").bfloat16() for _ in range(2))
+    table = (torch.arange(n, device="cuda") % 3).to(torch.int32).view(n, 1)
+    lens = torch.ones(n, dtype=torch.int32, device="cuda")
+    q, out = torch.randn(n, D, device="cuda").bfloat16(), torch.empty(n, D, device="cuda", dtype=torch.bfloat16)
+    assert _decode(q, D, kc, vc, table, lens, out, Hq, 1, D, 16, splits) == 0
+    assert torch.equal(out, vc[table[:, 0].long(), 0, 0])             # one key each

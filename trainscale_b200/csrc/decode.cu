@@ -115,6 +115,12 @@ __device__ __forceinline__ float high_part(float x) { return __uint_as_float(__f
 // and what they leave, at least `least`
 __device__ __forceinline__ float rest_part(float x, float least) { return fmaxf(x - high_part(x), least); }
 __device__ __forceinline__ uint32_t pack_high(float x, float y) { return __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632); }
+// eight values of a row of any alignment (query rows may be anybody's; caches are whole 16-byte vectors)
+__device__ __forceinline__ uint4 load_row8(const __nv_bfloat16* p) {
+  if ((reinterpret_cast<uintptr_t>(p) & 15u) == 0) return *reinterpret_cast<const uint4*>(p);
+  const uint16_t* h = reinterpret_cast<const uint16_t*>(p);
+  return make_uint4(h[0] | h[1] << 16, h[2] | h[3] << 16, h[4] | h[5] << 16, h[6] | h[7] << 16);
+}
 __device__ __forceinline__ void put_float4(float* dst, const float* v) { *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]); }
 
 // grid (splits, Hkv, sequences).  A CTA takes an even share of one sequence's keys for one kv head and all query heads that share
@@ -161,7 +167,7 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, const
   uint4 qv[NK];
 #pragma unroll
   for (int i = 0; i < NK; ++i)
-    qv[i] = head < group ? *reinterpret_cast<const uint4*>(q + static_cast<size_t>(seq) * q_stride + (hk * group + head) * D + i * 32 + tig * 8)
+    qv[i] = head < group ? load_row8(q + static_cast<size_t>(seq) * q_stride + (hk * group + head) * D + i * 32 + tig * 8)
                          : make_uint4(0u, 0u, 0u, 0u);
   float m = -INFINITY, l = 0.f;            // of the lane's head; l of this lane's keys
   float acc[NV * 8][4];                    // [n]: columns 2 tig, 2 tig + 1 <-> dimensions 64 (n / 8) + 8 column + n % 8
@@ -494,19 +500,24 @@ extern "C" int ts_decode_attention_ex(const void* q, int q_stride, const void* k
                                       int D, int block_size, int chunk, int splits, float scale, int window, float softcap,
                                       void* stream) {
   if (num_seqs <= 0) return 0;
-  if (Hkv <= 0 || Hq % Hkv != 0 || Hq / Hkv > DEC_MAX_GROUP || (D != 64 && D != 128) || splits <= 0 || num_seqs > 65535 ||
-      Hkv > 65535)
+  if (Hkv <= 0 || Hq % Hkv != 0 || Hq / Hkv > DEC_MAX_GROUP || (D != 64 && D != 128) || splits <= 0 || Hkv > 65535)
     return -10;
-  if (q_stride % 8 || (reinterpret_cast<uintptr_t>(q) & 15u)) return -11;
+  if ((reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15u) return -11;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const float log2e = 1.4426950408889634f;
   const bool cluster = splits <= DEC_MAX_CLUSTER;
   const bool ext = window > 0 || softcap > 0.f, wide = Hq / Hkv > 4;
   auto launch = D == 128 ? (cluster ? pick_decode<128, true>(ext, wide) : pick_decode<128, false>(ext, wide))
                          : (cluster ? pick_decode<64, true>(ext, wide) : pick_decode<64, false>(ext, wide));
-  const int rc = launch(q, q_stride, k_cache, v_cache, block_table, max_blocks, seq_lens, out, out_stride, part_out, part_lse,
-                        num_seqs, Hq, Hkv, block_size, chunk, splits, scale * log2e, window, softcap > 0.f ? scale / softcap : 0.f,
-                        softcap > 0.f ? softcap * log2e : 0.f, st);
+  int rc = 0;
+  for (int s0 = 0; s0 < num_seqs && !rc; s0 += 65535) {          // the grid's third dimension ends there
+    const size_t part = static_cast<size_t>(s0) * Hq * splits;
+    rc = launch((const __nv_bfloat16*)q + static_cast<size_t>(s0) * q_stride, q_stride, k_cache, v_cache,
+                block_table + static_cast<size_t>(s0) * max_blocks, max_blocks, seq_lens + s0,
+                (__nv_bfloat16*)out + static_cast<size_t>(s0) * out_stride, out_stride, cluster ? nullptr : part_out + part * D,
+                cluster ? nullptr : part_lse + part, num_seqs - s0 < 65535 ? num_seqs - s0 : 65535, Hq, Hkv, block_size, chunk, splits,
+                scale * log2e, window, softcap > 0.f ? scale / softcap : 0.f, softcap > 0.f ? softcap * log2e : 0.f, st);
+  }
   if (rc || cluster) return rc;
   if (D == 128)
     decode_merge_kernel<128><<<dim3(num_seqs, Hq), 128, 0, st>>>(part_out, part_lse, (__nv_bfloat16*)out, out_stride, Hq, splits);
