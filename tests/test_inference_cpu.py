@@ -293,3 +293,23 @@ def test_decode_splits_leave_no_long_share():
                 assert s >= 1 and -(-longest // s) <= 12288 and (s == 1 or longest // s >= 128), (n, heads, longest, s)
                 if longest <= 12288:
                     assert s <= max(1, -(-256 // (n * heads)))         # even batches fill the GPU once
+
+
+def test_only_a_step_fetches_weights_ahead(monkeypatch):
+    """`logits` and the norm of step rows, called on their own, may follow the kernel that wrote their weight: only the calls inside a
+    step, behind the launch of its embedding, ask for weights before their turn."""
+    from trainscale_b200.inference import engine as E
+    core, model = _core(32)
+    asked = []
+
+    def product(x, w, out_dtype=None, chained=False):
+        asked.append(chained)
+        y = x @ w.t()
+        return y if out_dtype is None else y.to(out_dtype)
+
+    monkeypatch.setattr(E.gemm, "step_linear", product)
+    core.runner.cuda = True                                       # (the dispatch of the GPU path; the product is the one above)
+    core.runner.logits(torch.zeros(2, CFG.hidden_size))
+    assert asked == [False]
+    import inspect
+    assert inspect.signature(E.norm.rmsnorm_step).parameters["chained"].default is False

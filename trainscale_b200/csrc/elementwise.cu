@@ -1125,11 +1125,11 @@ extern "C" int ts_rmsnorm_fwd(const void* x, const void* residual, const void* w
   return (int)cudaGetLastError();
 }
 
-// The same for the rows of a serving step, H <= 8192: no rstd, chained launch (w as the weights of launch_chained).
+// The same for the rows of a serving step, H <= 8192: no rstd; chained: see launch_chained (w is one of its weights).
 extern "C" int ts_rmsnorm_step(const void* x, const void* residual, const void* w, void* y, void* res_out, long long rows, int H,
-                               float eps, float w_offset, void* stream) {
+                               float eps, float w_offset, int chained, void* stream) {
   if (H % 8 != 0 || H <= 0 || H > 8192 || rows <= 0 || rows > 0x7fffffffll) return -10;
-  return launch_chained(rmsnorm_step_kernel, dim3((unsigned)rows), dim3((unsigned)((H / 8 + 31) / 32 * 32)), 0, ST(stream), 1, true,
+  return launch_chained(rmsnorm_step_kernel, dim3((unsigned)rows), dim3((unsigned)((H / 8 + 31) / 32 * 32)), 0, ST(stream), 1, chained != 0,
                         (const bf16*)x, (const bf16*)residual, (const bf16*)w, (bf16*)y, (bf16*)res_out, H, eps, w_offset);
 }
 

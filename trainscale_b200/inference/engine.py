@@ -304,7 +304,7 @@ class ModelRunner:
 
     def _norm(self, module, x: torch.Tensor, res: torch.Tensor | None):
         if self.cuda and type(module) is RMSNorm:
-            return norm.rmsnorm_step(x, module.weight, module.eps, res, module.offset)
+            return norm.rmsnorm_step(x, module.weight, module.eps, res, module.offset, chained=True)
         return module(x, res)
 
     def _rotate_and_cache(self, layer: int, qkv: torch.Tensor, batch: StepBatch) -> torch.Tensor:
@@ -520,7 +520,7 @@ class ModelRunner:
         st = {"batch": batch, "host": views(host_arena), "arena": arena, "host_arena": host_arena, "copied": torch.cuda.Event()}
 
         def body():
-            return self.logits(self._layers(batch))
+            return self.logits(self._layers(batch), chained=True)
 
         side = torch.cuda.Stream(device=dev)
         side.wait_stream(torch.cuda.current_stream())
@@ -535,11 +535,12 @@ class ModelRunner:
         return st
 
     @torch.no_grad()
-    def logits(self, hidden: torch.Tensor) -> torch.Tensor:
-        """fp32 logits of hidden states [n, H]."""
+    def logits(self, hidden: torch.Tensor, chained: bool = False) -> torch.Tensor:
+        """fp32 logits of hidden states [n, H].  `chained`: directly behind the layers of the same step (gemm.step_linear); a call of
+        its own may follow whatever wrote the head's weight, so it waits for it."""
         if self.own_layers or self.tp is not None or not self.cuda:
             return self.model.logits(hidden).float()
-        z, cap = gemm.step_linear(hidden, self.model.head_weight, torch.float32, chained=True), self.cfg.final_logit_softcap
+        z, cap = gemm.step_linear(hidden, self.model.head_weight, torch.float32, chained=chained), self.cfg.final_logit_softcap
         return cap * torch.tanh(z / cap) if cap and cap > 0 else z
 
 
@@ -725,7 +726,7 @@ class EngineCore:
             hidden = self.runner.forward(host.to_device(self.device, self.runner.lora is not None))
             if not host.out_rows:
                 return None
-            logits = self.runner.logits(hidden)
+            logits = self.runner.logits(hidden, chained=True)
         if host.out_entry != sorted(host.out_entry):
             logits = logits[torch.tensor(sorted(range(len(host.out_entry)), key=lambda i: host.out_entry[i]),
                                          device=self.device)]

@@ -104,9 +104,10 @@ STEP_ROWS = 1024     # rows up to which a CTA per row (ts_rmsnorm_step) is taken
 
 
 @torch.no_grad()
-def rmsnorm_step(x: torch.Tensor, w: torch.Tensor, eps: float, residual: torch.Tensor | None = None, w_offset: float = 0.0):
-    """`rmsnorm` of the rows of a serving step, without autograd.  `w` may be fetched while the kernels before this one still run,
-    back to the last ordinary launch: none of these may be what writes it."""
+def rmsnorm_step(x: torch.Tensor, w: torch.Tensor, eps: float, residual: torch.Tensor | None = None, w_offset: float = 0.0,
+                 chained: bool = False):
+    """`rmsnorm` of the rows of a serving step, without autograd.  `chained`: `w` may be fetched while the kernels before this one
+    still run, back to the last ordinary launch, so none of these may be what writes it."""
     H = x.shape[-1]
     if not (x.is_cuda and x.dtype == w.dtype == torch.bfloat16 and H % 8 == 0 and H <= 8192 and x.dim() == 2
             and 0 < x.shape[0] <= STEP_ROWS and (residual is None or residual.shape == x.shape and residual.dtype == x.dtype)
@@ -116,7 +117,8 @@ def rmsnorm_step(x: torch.Tensor, w: torch.Tensor, eps: float, residual: torch.T
     res = x if residual is None else torch.empty_like(x)
     rc = _lib.load("elementwise").ts_rmsnorm_step(
         _lib.ptr(x), _lib.ptr(residual), _lib.ptr(w), _lib.ptr(y), _lib.ptr(None if residual is None else res),
-        ctypes.c_longlong(x.shape[0]), H, ctypes.c_float(eps), ctypes.c_float(w_offset), _lib.stream_ptr())
+        ctypes.c_longlong(x.shape[0]), H, ctypes.c_float(eps), ctypes.c_float(w_offset), int(chained),
+        _lib.stream_ptr())
     _lib.check(rc, "ts_rmsnorm_step")
     return y, res
 
