@@ -313,3 +313,44 @@ def test_only_a_step_fetches_weights_ahead(monkeypatch):
     assert asked == [False]
     import inspect
     assert inspect.signature(E.norm.rmsnorm_step).parameters["chained"].default is False
+
+
+def test_hooks_and_overrides_count_where_step_kernels_would_pass_them_by(monkeypatch):
+    """A norm with hooks or a forward of its own is called as a module, a model with other logits is asked for them."""
+    import pytest
+    from trainscale_b200.inference import engine as E
+    from trainscale_b200.models.llama import LlamaForCausalLM
+    core, model = _core(32)
+    runner, norm = core.runner, model.model.norm
+    runner.cuda = True                                            # (the dispatch of the GPU path, whose kernels must not be reached)
+
+    def kernel(*a, **k):
+        raise AssertionError("step kernel")
+
+    monkeypatch.setattr(E.norm, "rmsnorm_step", kernel)
+    monkeypatch.setattr(E.gemm, "step_linear", kernel)
+    x = torch.randn(3, CFG.hidden_size)
+    with pytest.raises(AssertionError, match="step kernel"):
+        runner._norm(norm, x, None)
+    seen = []
+    for register in (norm.register_forward_hook, norm.register_forward_pre_hook,
+                     torch.nn.modules.module.register_module_forward_hook):
+        handle = register(lambda m, *a: seen.append(m))
+        runner._norm(norm, x, None)
+        handle.remove()
+    assert seen == [norm] * 3
+    monkeypatch.setattr(norm, "forward", lambda x, res=None: (x + 1, x))
+    assert torch.equal(runner._norm(norm, x, None)[0], x + 1)
+
+    class Scaled(LlamaForCausalLM):
+        def logits(self, hidden):
+            return 2 * super().logits(hidden)
+
+    with pytest.raises(AssertionError, match="step kernel"):
+        runner.logits(x)
+    want = 2 * model.logits(x)
+    model.__class__ = Scaled
+    assert torch.allclose(runner.logits(x), want)
+    model.__class__ = LlamaForCausalLM
+    monkeypatch.setattr(model, "logits", lambda h: h * 3)
+    assert torch.equal(runner.logits(x), x * 3)

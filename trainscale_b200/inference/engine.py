@@ -24,11 +24,12 @@ from dataclasses import asdict, dataclass, field
 from typing import Any, AsyncIterator, Iterable
 
 import torch
+from torch.nn.modules.module import _has_any_global_hook
 
 from ..utils.refargs import ANY, reference_kwargs
 
 from ..core.types import Err, Ok, Result
-from ..models.llama import RMSNorm
+from ..models.llama import LlamaForCausalLM, RMSNorm
 from ..ops import _lib, activation, attention, flash, gemm, norm, rope
 from .batch import HostBatch, StepBatch, StepEntry
 from .kv_cache import CacheSpec, PagedKVCache
@@ -303,7 +304,8 @@ class ModelRunner:
         return y
 
     def _norm(self, module, x: torch.Tensor, res: torch.Tensor | None):
-        if self.cuda and type(module) is RMSNorm:
+        if self.cuda and type(module) is RMSNorm and not (module._forward_hooks or module._forward_pre_hooks or
+                                                          "forward" in module.__dict__ or _has_any_global_hook()):
             return norm.rmsnorm_step(x, module.weight, module.eps, res, module.offset, chained=True)
         return module(x, res)
 
@@ -538,7 +540,8 @@ class ModelRunner:
     def logits(self, hidden: torch.Tensor, chained: bool = False) -> torch.Tensor:
         """fp32 logits of hidden states [n, H].  `chained`: directly behind the layers of the same step (gemm.step_linear); a call of
         its own may follow whatever wrote the head's weight, so it waits for it."""
-        if self.own_layers or self.tp is not None or not self.cuda:
+        if self.own_layers or self.tp is not None or not self.cuda or "logits" in self.model.__dict__ or \
+                getattr(type(self.model), "logits", None) is not LlamaForCausalLM.logits:
             return self.model.logits(hidden).float()
         z, cap = gemm.step_linear(hidden, self.model.head_weight, torch.float32, chained=chained), self.cfg.final_logit_softcap
         return cap * torch.tanh(z / cap) if cap and cap > 0 else z
