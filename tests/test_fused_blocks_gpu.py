@@ -140,3 +140,68 @@ def test_embedding_gradient_in_the_owners_rows(ids, H, added):
     del w.main_grad
     emb(flat.view(1, -1)).backward(dy)                 # without an owner: torch's own gradient
     assert w.grad is not None
+
+
+def _owned_embedding(V=40, H=16):
+    from trainscale_b200.ops.embedding import TokenEmbedding
+    torch.manual_seed(0)
+    emb = TokenEmbedding(V, H).to("cuda", torch.bfloat16)
+    emb.weight._ts_unit, emb.weight.grad_added = object(), False
+    emb.weight.main_grad = torch.full((V, H), 3.0, device="cuda")
+    ids = torch.randint(0, V, (2, 9), device="cuda")
+    return emb, ids, torch.randn(2, 9, H, device="cuda").bfloat16()
+
+
+def _dense(emb, ids, dy):
+    return torch.zeros_like(emb.weight.main_grad).index_add(0, ids.reshape(-1), dy.reshape(-1, dy.shape[-1]).float())
+
+
+def test_embedding_weight_may_change_before_its_gradient():
+    emb, ids, dy = _owned_embedding()
+    y = emb(ids)
+    with torch.no_grad():
+        emb.weight.mul_(2)
+    y.backward(dy)
+    assert emb.weight.grad_added and torch.allclose(emb.weight.main_grad, _dense(emb, ids, dy), atol=1e-5)
+
+
+@pytest.mark.parametrize("when", ["before", "between"])
+@pytest.mark.parametrize("kind", ["register_hook", "register_post_accumulate_grad_hook"])
+def test_hooks_see_the_embedding_gradient(when, kind):
+    emb, ids, dy = _owned_embedding()
+    seen, w = [], emb.weight
+    hook = (lambda g: seen.append(g.clone())) if kind == "register_hook" else (lambda p: seen.append(p.grad.clone()))
+    if when == "before":
+        getattr(w, kind)(hook)
+    y = emb(ids)
+    if when == "between":
+        getattr(w, kind)(hook)
+    y.backward(dy)
+    # the same gradient in bf16 (2^-8 of sums of a few unit values)
+    assert len(seen) == 1 and torch.allclose(seen[0].float(), _dense(emb, ids, dy), atol=2e-2)
+    assert torch.equal(w.grad, seen[0]) and not w.grad_added and (w.main_grad == 3.0).all()
+
+
+def test_embedding_gradients_that_are_asked_for():
+    """`torch.autograd.grad` returns the weight's gradient, once and again, and one of something else leaves the owner's alone."""
+    emb, ids, dy = _owned_embedding()
+    (g,) = torch.autograd.grad(emb(ids), emb.weight, dy)
+    assert torch.allclose(g.float(), _dense(emb, ids, dy), atol=2e-2)
+    scale = torch.ones((), device="cuda", requires_grad=True)
+    torch.autograd.grad((emb(ids) * scale).float().sum(), scale)
+    assert not emb.weight.grad_added and (emb.weight.main_grad == 3.0).all()
+    # d/ds of sum(g * m), where g = s * (gradient for dy)
+    (g,) = torch.autograd.grad(emb(ids) * scale, emb.weight, dy, create_graph=True)
+    (d,) = torch.autograd.grad(g.float().sum(), scale)
+    assert abs(float(d) - float(dy.float().sum())) <= 0.02 * float(dy.float().abs().sum())
+
+
+def test_embedding_under_transforms():
+    emb, ids, dy = _owned_embedding()
+    want = torch.nn.functional.embedding(ids, emb.weight)
+    assert torch.equal(torch.func.vmap(emb)(ids), want)
+    t = torch.randn_like(emb.weight)
+    with torch.autograd.forward_ad.dual_level():
+        w = torch.autograd.forward_ad.make_dual(emb.weight, t)
+        out = torch.func.functional_call(emb, {"weight": w}, (ids,))
+        assert torch.equal(torch.autograd.forward_ad.unpack_dual(out).tangent, t[ids])
