@@ -48,6 +48,7 @@ struct GemmParams {
   float act_a, act_b;       // its constants
   int act_cols;             // columns it applies to, from the first; a multiple of 32 unless all
   int tma_c;                // results leave by TMA
+  int c_rows;               // rows of C in all
 };
 
 constexpr int GEMM_EP_BYTES = 4 * 2 * 4096;   // two 32-row x 64-column staging tiles per epilogue warp
@@ -176,6 +177,16 @@ __device__ __forceinline__ void gemm_store_tma(const GemmParams& p, const CUtens
     if (p.act != 0) {
       gemm_activate(p, r, col0);
       gemm_activate(p, r + 32, col0 + 32);
+    }
+    // A store that the map clips still writes whole 16-byte pieces: zeros beside a last column that is no multiple of eight.  Those
+    // columns are stored directly.
+    const int rows = min(32, p.c_rows - row0), cols = min(64, p.N - col0);
+    if (cols & 7) {
+      if (lane < rows) {
+        gemm_store_chunk(p, r, static_cast<size_t>(row0 + lane), col0);
+        if (cols > 32) gemm_store_chunk(p, r + 32, static_cast<size_t>(row0 + lane), col0 + 32);
+      }
+      continue;
     }
     uint8_t* buf = stage + (issued & 1u) * 4096;
     if (lane == 0) tma_store_wait_read<1>();
@@ -660,6 +671,7 @@ static bool glu_ok(int act, const void* C, int N, int ldc, int out_fp32) {
 static void plan_result(CUtensorMap& tmC, const CUtensorMap& unused, GemmParams& p, int slabs) {
   tmC = unused;
   p.tma_c = 0;
+  p.c_rows = slabs * p.M;
 #ifndef TS_DEBUG
   if (p.out_fp32 || p.accumulate || p.act >= ACT_FIRST_GLU || (slabs > 1 && p.M % GEMM_BM) || p.ldc % 8 ||
       (reinterpret_cast<uintptr_t>(p.C) & 15u) || p.ldc < p.N)
