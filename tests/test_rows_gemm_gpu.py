@@ -72,3 +72,18 @@ def test_every_route_of_the_dispatch(M, N, K):
     y = gemm.step_glu(x, w, "silu").double() - torch.nn.functional.silu(half) * ref[:, N // 2:]
     # two roundings of gate and up to bf16 where the product is not fused
     assert (y.abs() <= 2.0 ** -6 * (1 + half.abs()) * (1 + ref[:, N // 2:].abs())).all()
+
+
+@pytest.mark.parametrize("N,K", [(128, 64), (2048, 2048), (384, 8192), (64, 16384)])
+def test_fp32_results_and_partial_sums_keep_fp32(N, K):
+    """Relative to the norm of the result: K products added in fp32, a bit of 2^-24 lost at random (or, as tensor cores add, always
+    towards zero: 2^-24 for each of the K / 16 steps) stays below 1e-5 * max(1, K / 2048).  bf16 anywhere, in the result or in the
+    partial sums of a split reduction, would leave 2^-9 / sqrt(3) = 1.1e-3."""
+    torch.manual_seed(0)
+    w = torch.randn(N, K, device="cuda").bfloat16()
+    for M in (1, 16, 97, 256):
+        x = torch.randn(M, K, device="cuda").bfloat16()
+        y, ref = _run(x, w, N, torch.float32), _exact(x, w)
+        err, bound = float((y.double() - ref).norm() / ref.norm()), 1e-5 * max(1.0, K / 2048)
+        assert err <= bound, (M, err)
+        assert float((y.bfloat16().double() - ref).norm() / ref.norm()) > 10 * bound          # the bound would see it
