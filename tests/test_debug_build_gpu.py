@@ -12,7 +12,7 @@ ROOT = Path(__file__).resolve().parent.parent
 
 
 def _run(code: str, **env) -> str:
-    e = dict(os.environ, TS_DEBUG="1", PYTHONPATH=str(ROOT), **env)
+    e = {**os.environ, "TS_DEBUG": "1", "PYTHONPATH": str(ROOT), **env}
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=600, env=e, cwd=str(ROOT))
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-3000:]
     return r.stdout
@@ -91,3 +91,42 @@ else:
 dist.destroy_process_group()
 """)
     assert "CAUGHT" in out or "NO_SYMM" in out
+
+
+def test_debug_build_runs_the_stores_that_ship():
+    """Results that leave by TMA, all tiles and both grouped modes, and the streamed products: the release build's bits, nothing beside
+    them written, nothing reported."""
+    code = """
+import torch
+from trainscale_b200.ops import _lib, build, gemm, moe
+assert build.DEBUG == {debug}
+torch.manual_seed(0)
+out = []
+def rand(*shape):
+    return torch.randn(*shape, device="cuda").bfloat16()
+def room(rows, cols):
+    wide = torch.full((rows + 40, cols + 72), 7.0, device="cuda", dtype=torch.bfloat16)
+    out.append(wide)
+    return wide[:rows, 8:8 + cols]
+for bn, M, N, K in ((64, 33, 72, 64), (128, 300, 200, 136), (256, 261, 328, 64), (512, 521, 328, 72)):
+    gemm.matmul_nt(rand(M, K), rand(N, K), out=room(M, N), bn=bn)
+gemm._stream_rows(rand(97, 200), rand(130, 200), 130, torch.float32, -1)
+groups = torch.tensor([0, -1, 1], dtype=torch.int32, device="cuda")
+moe._grouped(1, rand(384, 64), rand(2, 200, 64), room(384, 200), 384, 200, 64, 64, 64, 272, False, False, False, groups, 2)
+seg = torch.tensor([0, 128, 128, 384], dtype=torch.int32, device="cuda")
+moe._grouped(2, rand(384, 256), rand(384, 200), room(768, 200), 256, 200, 384, 256, 200, 272, True, True, False, seg, 3)
+torch.cuda.synchronize()
+_lib.raise_on_any_device_error()
+torch.save([t.cpu() for t in out], {path!r})
+print("CLEAN")
+"""
+    import torch
+    got = []
+    for debug in (True, False):
+        path = f"/tmp/ts_stores_{os.getpid()}_{int(debug)}.pt"
+        assert "CLEAN" in _run(code.format(debug=debug, path=path), **({} if debug else {"TS_DEBUG": "0"}))
+        got.append(torch.load(path))
+        os.unlink(path)
+    assert len(got[0]) == 6 and all(torch.equal(a, b) for a, b in zip(*got))
+    for wide in got[0]:
+        assert (wide[-40:] == 7.0).all() and (wide[:, :8] == 7.0).all() and (wide[:, -64:] == 7.0).all()

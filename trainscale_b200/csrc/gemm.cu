@@ -181,7 +181,12 @@ __device__ __forceinline__ void gemm_store_tma(const GemmParams& p, const CUtens
     // A store that the map clips still writes whole 16-byte pieces: zeros beside a last column that is no multiple of eight.  Those
     // columns are stored directly.
     const int rows = min(32, p.c_rows - row0), cols = min(64, p.N - col0);
-    if (cols & 7) {
+    bool direct = (cols & 7) != 0;
+#ifdef TS_DEBUG
+    // the tile against C's extent: one that reaches beyond goes row by row, whose check skips and reports
+    direct |= (static_cast<size_t>(row0 + rows - 1) * p.ldc + col0 + cols) * 2 > p.c_bytes;
+#endif
+    if (direct) {
       if (lane < rows) {
         gemm_store_chunk(p, r, static_cast<size_t>(row0 + lane), col0);
         if (cols > 32) gemm_store_chunk(p, r + 32, static_cast<size_t>(row0 + lane), col0 + 32);
@@ -666,19 +671,17 @@ static bool glu_ok(int act, const void* C, int N, int ldc, int out_fp32) {
   return act < ACT_FIRST_GLU || (N % (2 * GLU_BLOCK) == 0 && !out_fp32 && ldc % 8 == 0 && ldc >= N / 2 &&
                                  (reinterpret_cast<uintptr_t>(C) & 15u) == 0);
 }
-// Map of a bf16 result that TMA can store: p.tma_c and true, or direct stores (`tmC` is then unused).  The debug build checks every
-// store against C's extent, so it keeps the direct ones.  Slabs of a grouped reduction must end on a tile's border.
+// Map of a bf16 result that TMA can store (p.tma_c), or direct stores (`tmC` is then unused).  Slabs of a grouped reduction must end
+// on a tile's border.
 static void plan_result(CUtensorMap& tmC, const CUtensorMap& unused, GemmParams& p, int slabs) {
   tmC = unused;
   p.tma_c = 0;
   p.c_rows = slabs * p.M;
-#ifndef TS_DEBUG
   if (p.out_fp32 || p.accumulate || p.act >= ACT_FIRST_GLU || (slabs > 1 && p.M % GEMM_BM) || p.ldc % 8 ||
       (reinterpret_cast<uintptr_t>(p.C) & 15u) || p.ldc < p.N)
     return;
   p.tma_c = make_tmap_2d(&tmC, p.C, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)slabs * p.M, (uint64_t)p.N, (uint64_t)p.ldc, 32,
                          64) == 0;
-#endif
 }
 static int result_cols(int act, int N) { return act >= ACT_FIRST_GLU ? N / 2 : N; }
 

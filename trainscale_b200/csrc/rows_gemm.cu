@@ -27,6 +27,7 @@ struct RowsGemmParams {
   int mt;                   // token rows of a CTA: M rounded up to 16, at most RG_TOKENS
   int stages, k_blocks, splits;
   void* out;
+  size_t out_bytes;         // extent of the result (debug build)
   long long ldo;
   int out_fp32;
 };
@@ -212,6 +213,7 @@ rows_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     const float f[4] = {v.x, v.y, v.z, v.w};
     if (p.out_fp32) {
       float* dst = reinterpret_cast<float*>(p.out) + (m0 + t) * p.ldo + n;
+      if (!TS_IN_BOUNDS(dst, min(4, p.N - n) * 4, p.out, p.out_bytes, 7200)) continue;
       if (n + 4 <= p.N && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
         *reinterpret_cast<float4*>(dst) = v;
       } else {
@@ -221,6 +223,7 @@ rows_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       }
     } else {
       __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.out) + (m0 + t) * p.ldo + n;
+      if (!TS_IN_BOUNDS(dst, min(4, p.N - n) * 2, p.out, p.out_bytes, 7200)) continue;
       if (n + 4 <= p.N && (reinterpret_cast<uintptr_t>(dst) & 7u) == 0) {
         *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
       } else {
@@ -266,6 +269,7 @@ extern "C" int ts_rows_gemm(const void* X, const void* W, void* out, int M, int 
   if (M <= 0 || N <= 0 || K <= 0 || glu > 2) return -10;
   RowsGemmParams p;
   p.M = M; p.N = N; p.K = K; p.out = out; p.ldo = ldo; p.out_fp32 = out_fp32;
+  p.out_bytes = (static_cast<size_t>(M - 1) * ldo + N) * (out_fp32 ? 4 : 2);
   p.mt = M > RG_TOKENS ? RG_TOKENS : (M + 15) / 16 * 16;
   p.k_blocks = (K + 63) / 64;
   const int cols = glu >= 0 ? 64 : 128, tiles = (N + cols - 1) / cols, blocks = (M + RG_TOKENS - 1) / RG_TOKENS;
