@@ -354,3 +354,14 @@ def test_hooks_and_overrides_count_where_step_kernels_would_pass_them_by(monkeyp
     model.__class__ = LlamaForCausalLM
     monkeypatch.setattr(model, "logits", lambda h: h * 3)
     assert torch.equal(runner.logits(x), x * 3)
+
+
+def test_a_step_looks_for_its_longest_row_once():
+    from trainscale_b200.inference.batch import HostBatch, StepEntry
+    core, _ = _core(64)
+    core.execute([StepEntry(0, [1] * 20, []), StepEntry(1, [2] * 5, [])])
+    host = HostBatch(core.cache, [StepEntry(0, [3]), StepEntry(1, [4]), StepEntry(2, [5] * 30)])
+    batch = host.to_device("cpu")
+    assert batch.longest_single == 21
+    host.starts = None                                    # every layer asks; the lists are not walked again
+    assert batch.longest_single == 21

@@ -176,13 +176,16 @@ class StepBatch:
     @property
     def all_wanted(self) -> bool:
         """Logits of every row, in order, are asked for (a captured decode always does)."""
-        return self.host is None or self.host.out_rows == list(range(self.num_tokens))
+        h = self.host
+        return h is None or len(h.out_rows) == self.num_tokens and h.out_rows == list(range(self.num_tokens))
 
     @property
     def longest_single(self) -> int:
-        """Upper bound of the keys that a single-token entry sees."""
-        h = self.host
-        return self.max_len if h is None else max(s + 1 for s in h.starts[:self.n_single])
+        """Upper bound of the keys that a single-token entry sees (every layer asks)."""
+        if "longest_single" not in self._contexts:
+            h = self.host
+            self._contexts["longest_single"] = self.max_len if h is None else max(s + 1 for s in h.starts[:self.n_single])
+        return self._contexts["longest_single"]
 
     def key_groups(self, limit: int) -> list[KeyGroup]:
         """The multi-token entries in groups of at most `limit` key rows (or of one entry), uploaded once per step."""
