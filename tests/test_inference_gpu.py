@@ -491,3 +491,19 @@ def test_decode_attention_of_more_sequences_than_a_grid_has(splits):
     q, out = torch.randn(n, D, device="cuda").bfloat16(), torch.empty(n, D, device="cuda", dtype=torch.bfloat16)
     assert _decode(q, D, kc, vc, table, lens, out, Hq, 1, D, 16, splits) == 0
     assert torch.equal(out, vc[table[:, 0].long(), 0, 0])             # one key each
+
+
+@pytest.mark.parametrize("design,shape", [("lovurax", dict(kv=1)), ("mezilix", dict(experts=4, top=2))])
+def test_the_serving_benchmarks_closest_table_covers_the_step(design, shape):
+    """Every function that the table of the closest model times is called by a prompt's step and by a decoding one."""
+    from trainscale_b200.inference import bench_serving as S
+    from trainscale_b200.inference.batch import HostBatch, StepEntry
+    z = dict(width=256, layers=2, heads=4, dim=64, ff=384, **shape)
+    core = S.make_core(S.DESIGNS[design].closest(z), 4096, 4)
+    for entries, lengths in (([StepEntry(0, list(range(300)))], [(0, 300)]), ([StepEntry(0, [1])], [(300, 1)])):
+        batch = HostBatch(core.cache, entries).to_device("cuda")
+        with S.OpTimer(S.closest_table(z, sum(n for _, n in lengths), lengths, core.runner)) as t, torch.no_grad():
+            core.runner.logits(core.runner.forward(batch))
+        assert t.missing == []
+        ops = t.summary({"hbm_gbs": 6460.0, "bf16_tflops": 1695.0})
+        assert {"rms norm", "rotary, cache write", "attention"} <= set(ops) and ops["rms norm"]["calls"] == 2 * 2 + 1

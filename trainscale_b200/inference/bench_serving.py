@@ -150,13 +150,13 @@ class OpTimer:
     `(bytes, tensor-core flops, fp32 flops)`."""
 
     def __init__(self, table: list[tuple]):
-        self.table, self.records, self.saved, self.depth = table, [], [], 0
+        self.table, self.records, self.saved, self.depth, self.called = table, [], [], 0, set()
 
     def __enter__(self):
         for owner, attr, name, cost in self.table:
             fn = getattr(owner, attr)
             self.saved.append((owner, attr, fn))
-            setattr(owner, attr, self._wrap(fn, name, cost))
+            setattr(owner, attr, self._wrap(fn, attr, name, cost))
         return self
 
     def __exit__(self, *exc):
@@ -164,10 +164,16 @@ class OpTimer:
             setattr(owner, attr, fn)
         self.saved.clear()
 
-    def _wrap(self, fn, name, cost):
+    @property
+    def missing(self) -> list[str]:
+        """Functions of the table that the measured calls never reached (or only inside others of it)."""
+        return [attr for _, attr, _, _ in self.table if attr not in self.called]
+
+    def _wrap(self, fn, attr, name, cost):
         def call(*a, **k):
             if self.depth:
                 return fn(*a, **k)
+            self.called.add(attr)
             self.depth += 1
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             e0.record()
@@ -421,7 +427,7 @@ def lovurax_table(z: dict, rows: int, lengths: list[tuple[int, int]]) -> list[tu
 
 
 def closest_table(z: dict, rows: int, lengths: list[tuple[int, int]], runner) -> list[tuple]:
-    from ..ops import activation, gemm, moe, norm, rope
+    from ..ops import activation, gemm, moe, norm
     W, H, D = z["width"], z["heads"], z.get("vdim") or z["dim"]
     keys, pairs = _seen(lengths, KeyMask(UNBOUNDED))
     hkv = z.get("kv") or max(1, H // 4)
@@ -430,12 +436,23 @@ def closest_table(z: dict, rows: int, lengths: list[tuple[int, int]], runner) ->
         E, N, K = a[1].shape
         return (_visited(z["top"], E, rows) * N * K * 2 + rows * z["top"] * (N + K) * 2, 2.0 * rows * z["top"] * N * K)
 
-    return [
-        (norm, "rmsnorm", "rms norm", lambda a, k, o: (_bytes(a[0], *[t for t in o if t is not None]) + _bytes(*a[3:4]), 0.0)),
-        (gemm, "linear", _linear_name("gemm"), _linear_cost),
-        (rope, "apply_rope_qkv", "rotary", lambda a, k, o: (2 * _bytes(a[0]) * (H + hkv) / (H + 2 * hkv), 0.0)),
-        (runner, "_write_cache", "cache write", lambda a, k, o: (2 * a[1].shape[0] * 2 * hkv * D * 2, 0.0)),
+    def norm_cost(a, k, out):
+        return _bytes(a[0], a[1], *a[3:4], out[0], *([out[1]] if out[1] is not a[0] else [])), 0.0
+
+    def glu_product_cost(a, k, out):
+        return _bytes(a[0], a[1], out), 2.0 * a[0].shape[0] * a[1].numel()
+
+    table = [
+        (norm, "rmsnorm_step", "rms norm", norm_cost),
+        (gemm, "step_linear", _linear_name("gemm"), _linear_cost),
+        # queries and keys rotated in place, keys and values to the cache
+        (runner, "_rotate_and_cache", "rotary, cache write",
+         lambda a, k, o: (2 * _bytes(a[1]) * (H + hkv) / (H + 2 * hkv) + 2 * a[1].shape[0] * 2 * hkv * D * 2, 0.0)),
         (runner, "_attend", "attention", lambda a, k, o: (keys * 2 * hkv * D * 2 + 2 * _bytes(o), 4.0 * pairs * H * D)),
+    ]
+    if "experts" not in z:
+        return table + [(gemm, "step_glu", lambda a, o: f"gated gemm {a[1].shape[0]}x{a[1].shape[1]}", glu_product_cost)]
+    return table + [
         (moe, "topk_softmax", "router top-k", lambda a, k, o: (_bytes(a[0], *o), 0.0)),
         (moe, "make_plan", "routing plan", lambda a, k, o: (_bytes(a[0], o.dest, o.src_of_row), 0.0)),
         (moe, "_permute_raw", "permute", lambda a, k, o: (_bytes(a[0]) + a[1].n * W * 2, 0.0)),
@@ -477,6 +494,8 @@ def measure(design: str, name: str, peaks: dict, prompts: int = 2, prompt_len: i
             with OpTimer(table(rows, lengths)) as t:
                 torch.cuda._sleep(200_000_000)
                 step()
+            if kind == "closest" and t.missing:
+                raise RuntimeError(f"the table of the closest model lists what its step does not call: {t.missing}")
             return t.summary(peaks)
 
         # prefill: whole prompts in one step
@@ -507,7 +526,7 @@ def measure(design: str, name: str, peaks: dict, prompts: int = 2, prompt_len: i
                 core.execute([StepEntry(j, _tokens(context, 100 + j), []) for j in range(i, min(n, i + 4))])
             host = HostBatch(core.cache, [StepEntry(j, [j + 1]) for j in range(n)])
             batch = host.to_device("cuda")
-            step = lambda: core.runner.logits(core.runner.forward(batch))   # noqa: E731
+            step = lambda: core.runner.logits(core.runner.forward(batch), chained=True)   # noqa: E731
             d = {"ms": _timed(step, iters), "ops": profile(step, n, [(context, 1)] * n)}
             if core.runner.can_graph(host):
                 core.runner.decode_graphed(host)
