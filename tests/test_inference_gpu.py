@@ -507,3 +507,55 @@ def test_the_serving_benchmarks_closest_table_covers_the_step(design, shape):
         assert t.missing == []
         ops = t.summary({"hbm_gbs": 6460.0, "bf16_tflops": 1695.0})
         assert {"rms norm", "rotary, cache write", "attention"} <= set(ops) and ops["rms norm"]["calls"] == 2 * 2 + 1
+
+
+@pytest.mark.parametrize("D,keys", [(64, 40), (128, 700)])
+def test_rotation_and_decode_attention_wait_in_a_chain(D, keys):
+    """Projection, rotation with cache write, attention and output product launched as a chain, against the same kernels one by one:
+    each reads what the one before it wrote, the attention also the row that the rotation has just put into the cache."""
+    import ctypes
+    from trainscale_b200.ops import _lib, gemm, rope
+    torch.manual_seed(0)
+    Hq, Hkv, n, bs, H = 8, 2, 17, 16, 2048
+    lib, kw, blocks = _lib.load("decode"), Hkv * D, -(-keys // bs)
+    wqkv, wo = _scaled((Hq + 2 * Hkv) * D, H), _scaled(H, Hq * D)
+    cos, sin = rope.rope_tables(keys, D, device="cuda")
+    table = torch.arange(n * blocks, dtype=torch.int32, device="cuda").view(n, blocks)
+    lens = torch.full((n,), keys, dtype=torch.int32, device="cuda")
+    kc0, vc0 = (torch.randn(n * blocks, bs, Hkv, D, device="cuda").bfloat16() for _ in range(2))
+    x0 = torch.randn(n, H, device="cuda").bfloat16()
+    splits = lib.ts_decode_splits(n, Hkv, keys)
+    assert splits <= 8
+    steps = [(torch.full((n,), p, dtype=torch.int32, device="cuda"),
+              table[:, p // bs].long() * bs + p % bs) for p in range(keys - 12, keys)]
+    torch.cuda.synchronize()
+
+    def run(chained):
+        def turn():
+            if not chained:
+                torch.cuda.synchronize()
+
+        x, kc, vc = x0, kc0.clone(), vc0.clone()
+        for pos, slots in steps:
+            qkv = gemm.step_linear(x, wqkv, chained=chained)
+            turn()
+            assert lib.ts_rope_cache(_lib.ptr(qkv), ctypes.c_longlong(qkv.stride(0)), _lib.ptr(cos), _lib.ptr(sin), _lib.ptr(pos),
+                                     _lib.ptr(slots), _lib.ptr(kc), _lib.ptr(vc), ctypes.c_longlong(n), Hq, Hkv, D,
+                                     _lib.stream_ptr()) == 0
+            turn()
+            out = torch.empty(n, Hq * D, dtype=torch.bfloat16, device="cuda")
+            assert lib.ts_decode_attention(_lib.ptr(qkv), qkv.stride(0), _lib.ptr(kc), _lib.ptr(vc), _lib.ptr(table), blocks,
+                                           _lib.ptr(lens), _lib.ptr(out), Hq * D, _lib.ptr(None), _lib.ptr(None), n, Hq, Hkv, D, bs, 16,
+                                           splits, ctypes.c_float(1 / math.sqrt(D)), _lib.stream_ptr()) == 0
+            turn()
+            x = gemm.step_linear(out, wo, chained=chained)
+            turn()
+        return x, kc, vc
+
+    want = run(False)
+    for _ in range(5):
+        assert all(torch.equal(a, b) for a, b in zip(run(True), want))
+
+
+def _scaled(rows, cols):
+    return (torch.randn(rows, cols, device="cuda") / cols ** 0.5).bfloat16()
