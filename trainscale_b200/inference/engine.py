@@ -476,7 +476,7 @@ class ModelRunner:
         while n_pad < n:
             n_pad *= 2
         bt, sl = self.cache.block_table(host.seq_ids, None)
-        self.check_length(int(sl.max()))
+        self.check_length(max(host.pos) + 1)
         width = -(-bt.shape[1] // 32) * 32
         key = (n_pad, width)
         st = self.graphs.get(key)
