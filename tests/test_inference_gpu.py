@@ -559,3 +559,28 @@ def test_rotation_and_decode_attention_wait_in_a_chain(D, keys):
 
 def _scaled(rows, cols):
     return (torch.randn(rows, cols, device="cuda") / cols ** 0.5).bfloat16()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_an_infinite_value_stays_in_its_dimension_of_portions(D):
+    """Portions of prompts make no number of an infinite value's dimension, and every other one keeps its bits."""
+    from trainscale_b200.ops import flash
+    torch.manual_seed(0)
+    Hq, Hkv, n, m = 4, 2, 40, 200
+    kw, i32 = Hkv * D, dict(dtype=torch.int32, device="cuda")
+    q = torch.randn(n, Hq * D, device="cuda").bfloat16()
+    kv = torch.zeros(256, 2 * kw, device="cuda").bfloat16()
+    kv[:m] = torch.randn(m, 2 * kw, device="cuda").bfloat16()
+
+    def run():
+        out = torch.empty(n, Hq, D, device="cuda", dtype=torch.bfloat16)
+        flash.flash_portions(q, kv[:, :kw], kv[:, kw:], out.view(n, -1), Hq, Hkv, D, torch.tensor([0, n], **i32),
+                             torch.tensor([0], **i32), torch.tensor([m], **i32), n, 1 / math.sqrt(D))
+        return out
+
+    want = run()
+    kv[5, kw + 3] = math.inf                                       # of the first key head
+    got = run()
+    assert not got[:, :2, 3].isfinite().any()
+    got[:, :2, 3] = want[:, :2, 3]
+    assert torch.equal(got, want)
