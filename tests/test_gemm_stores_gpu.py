@@ -28,7 +28,8 @@ def _check(wide, got, ref, rows=None):
 # tiles of every width, the paired kernel (512) and the rule's own choice (0); rows around 32 and 128, columns around 64; results that
 # TMA can address (column 8) and that it cannot (column 3)
 @pytest.mark.parametrize("bn", [0, 64, 128, 256, 512])
-@pytest.mark.parametrize("M,N", [(1, 8), (31, 64), (33, 72), (127, 129), (261, 328), (513, 520)])
+@pytest.mark.parametrize("M,N", [(1, 8), (31, 64), (33, 72), (40, 72), (127, 129), (261, 328), (264, 200),
+                                 (513, 520), (520, 328)])
 @pytest.mark.parametrize("first", [8, 3])
 def test_dense_results_stay_in_their_place(bn, M, N, first):
     from trainscale_b200.ops import _lib, gemm

@@ -365,3 +365,22 @@ def test_a_step_looks_for_its_longest_row_once():
     assert batch.longest_single == 21
     host.starts = None                                    # every layer asks; the lists are not walked again
     assert batch.longest_single == 21
+
+
+def test_tables_whose_angles_depend_on_their_length_keep_the_declared_one():
+    """The default max_model_len is longer than some models' declared positions; scalings that look at the table's length must not
+    serve other angles for it than the model's own forward has."""
+    import pytest
+    from trainscale_b200.inference.batch import StepEntry
+    half = CFG.head_dim // 2
+    for scaling in (dict(rope_type="longrope", original_max_position_embeddings=64, short_factor=[1.0] * half,
+                         long_factor=[4.0] * half),
+                    dict(rope_type="dynamic_ntk", factor=4.0, original_max_position_embeddings=64)):
+        core, model = _core(256, max_position_embeddings=64, rope_scaling=scaling, initializer_range=0.2)
+        ids = torch.randint(0, CFG.vocab_size, (60,), generator=torch.Generator().manual_seed(2)).tolist()
+        core.execute([StepEntry(0, ids[:40], [])])
+        got = core.execute([StepEntry(0, ids[40:])])[0]
+        assert torch.allclose(got, model(torch.tensor([ids])).logits[0, -1], atol=1e-3, rtol=1e-3)
+        assert core.runner.cos.shape[0] == 64
+        with pytest.raises(ValueError, match="longer than the 64"):
+            core.execute([StepEntry(0, [1] * 5)])

@@ -277,7 +277,10 @@ class ModelRunner:
             self.use_graphs = bool(use_graphs) and self.device.type == "cuda"
         else:
             self.cuda = self.device.type == "cuda" and next(model.parameters()).dtype == torch.bfloat16
-            self.cos, self.sin = model.model.rope_tables(self.device, max(min(self.cfg.max_position_embeddings, 1 << 16), max_len))
+            declared, scaling = min(self.cfg.max_position_embeddings, 1 << 16), self.cfg.rope_scaling or {}
+            # (a longer table would turn every position of these by other angles: they end where the model says)
+            fixed = str(scaling.get("rope_type", scaling.get("type", ""))).lower() in rope.LENGTH_DEPENDENT
+            self.cos, self.sin = model.model.rope_tables(self.device, declared if fixed else max(declared, max_len))
             ws = self.tp.size if self.tp is not None else 1
             self.Hq, self.Hkv = self.cfg.num_attention_heads // ws, self.cfg.num_key_value_heads // ws
             self.use_graphs = bool(use_graphs) and self.cuda

@@ -64,6 +64,9 @@ def rope_inv_freq(dim: int, theta: float = 10000.0, scaling: str = "none", facto
     return inv.float()
 
 
+LENGTH_DEPENDENT = ("longrope", "dynamic_ntk")        # scalings whose angles depend on how many positions a table has
+
+
 def yarn_magnitude(factor: float) -> float:
     """Factor of cos and sin that goes with a YaRN stretch."""
     return 0.1 * math.log(factor) + 1.0
@@ -78,7 +81,7 @@ def longrope_attention_factor(max_pos: int, original_max_pos: int) -> float:
 def rope_tables(max_pos: int, dim: int, theta: float = 10000.0, device=None, **scaling) -> tuple[torch.Tensor, torch.Tensor]:
     """cos/sin tables, fp32 [max_pos, dim/2]."""
     attention_factor = scaling.pop("attention_factor", None)
-    if str(scaling.get("scaling", "")).lower() in ("longrope", "dynamic_ntk"):
+    if str(scaling.get("scaling", "")).lower() in LENGTH_DEPENDENT:
         scaling.setdefault("max_pos", max_pos)
     inv = rope_inv_freq(dim, theta, **scaling)
     ang = torch.outer(torch.arange(max_pos, dtype=torch.float32), inv)
