@@ -136,8 +136,9 @@ __device__ __forceinline__ void put_float4(float* dst, const float* v) { *reinte
 // Every warp walks its own 16-key tiles with a softmax state of its own; states meet in shared memory, then over the splits: up
 // to DEC_MAX_CLUSTER in distributed shared memory, more through partial results [seq][Hq][split][D] fp32 and lse
 // [seq][Hq][split] for decode_merge_kernel.
-// One warp per key with shuffled dot products / this (32 query heads of 8 kv heads, us; at the copy bandwidth): 64 sequences of
-// 300 keys of 64 75 / 14.5 (6.1), of 2000 keys of 128 571 / 96 (81), 4 of 10000 keys of 128 249 / 34 (25), 1 of 100 of 64 16 / 5.
+// One warp per key with shuffled dot products / this (32 query heads of 8 kv heads, us between events with nothing cached; at the
+// copy bandwidth): 64 sequences of 300 keys of 64 110 / 25.5 (6.1), of 2000 keys of 128 580 / 113 (81), 4 of 10000 keys of 128
+// 261 / 50 (25), 17 of 10000 779 / 132 (108), 1 of 97 of 64 27.7 / 10.2.
 // EXT: a window (the last `window` keys, 0: all) or a soft cap of the scores (cap_log2 * tanh(s * cap_inv), cap_log2 0: none).
 template <int D, bool CLUSTER, bool EXT, bool WIDE>
 __global__ void __launch_bounds__(DEC_WARPS * 32)
