@@ -132,7 +132,8 @@ __device__ __forceinline__ void put_float4(float* dst, const float* v) { *reinte
 //              registers, cut into three bf16 parts of eight bits each, which hold all of an fp32 weight.  No part of a weight is
 //              zero (2^-24 of it at least): an infinite value stays infinite in every product.  The heads use eight
 //              of the sixteen rows, so rows 8 - 15 take the second part; up to four heads are given twice (rows 4 - 7 repeat
-//              rows 0 - 3) and rows 4 - 7 take the third, more (WIDE) need a second product for it
+//              rows 0 - 3) and rows 4 - 7 take the third at no cost, more (WIDE) need a second product for it, 3 - 10 % of the
+//              time (8 heads per key head, 64 sequences: 2000 keys of 128 117.6 -> 120.8 us, 300 of 64 26.6 -> 28.7)
 // Every warp walks its own 16-key tiles with a softmax state of its own; states meet in shared memory, then over the splits: up
 // to DEC_MAX_CLUSTER in distributed shared memory, more through partial results [seq][Hq][split][D] fp32 and lse
 // [seq][Hq][split] for decode_merge_kernel.
